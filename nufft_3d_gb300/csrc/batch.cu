@@ -337,7 +337,7 @@ static void set_io(nufft3d_batch *b, int mode, const float2 *const *in, float2 *
         // grid reallocated between calls never leaves a stale map)
         g.tmap_ok = 0;
         g.tmaps = b->d_tmaps + 4 * v;
-        for (int lw = 1; lw < 4; ++lw)
+        for (int lw = 1; lw < 4 && !b->stored_h; ++lw)
             if (encode_gather_map(p, S.G, b->nc[v], 1 << lw, &b->h_tmaps[4 * v + lw])) g.tmap_ok |= 1 << lw;
         g.scale = mode == 2 ? (float)(1.0 / (double)p->nnz) : (float)(1.0 / std::sqrt((double)p->nnz));
         g.wsample = mode == 2 ? p->d : nullptr;
@@ -420,9 +420,17 @@ static int run_fft_chains(nufft3d_batch *b, bool forward, cudaStream_t s)
 
 static int run_interp(nufft3d_batch *b, bool gather, cudaStream_t s)
 {
+    if (gather && b->stored_h) {
+        // each volume's own persistent launch over its stored H
+        for (int v = 0; v < b->nvol; ++v) {
+            const BatchInterp &g = b->h_gat[v];
+            NUFFT_TRY(launch_gather(b->plans[v], g.in, g.out, g.nc, g.scale, g.wsample, s));
+        }
+        return NUFFT3D_SUCCESS;
+    }
     for (auto &g : b->igroups)
         NUFFT_TRY(launch_interp_batch(gather, g.cb, b->R, b->radial, gather ? b->gat : b->spr, g.tab, g.n, g.smem,
-                                      b->plans[0]->kb, b->work, b->plans[0]->sm_count, s, b->stored_h));
+                                      b->plans[0]->kb, b->work, b->plans[0]->sm_count, s));
     return NUFFT3D_SUCCESS;
 }
 
@@ -578,11 +586,9 @@ extern "C" int nufft3d_batch_create(nufft3d_plan *const *plans, const int *nc, i
             d.g = p->geom;
             d.kb = p->kb;
             d.cand = p->cand_desc;
-            d.tap_rows = p->tap_rows;
-            d.tap_ent = p->tap_ent;
             d.status = plan_status(p);  // timeouts are reported on the volume's plan
             if (v == 0) b->stored_h = true;
-            if (!p->tap_ent) b->stored_h = false;
+            if (!p->gw) b->stored_h = false;
             d.nc = nc[v];
             b->h_gat[v] = d;
             b->h_spr[v] = d;

@@ -178,11 +178,29 @@ struct InterpStatus {
     int polls;  // polls of each bounded wait
 };
 
+// A record of the stored-H gather: rows of four samples of one slab of a tile
+// (origin of the slab's first plane; planes not already in the ring when the
+// record before it was the previous one of the list).
+struct GatherRec {
+    int ox, oy, oz, nload;
+    uint32_t row0;
+    int nrows, s0, ns;
+    uint32_t chunk0, nchunk;  // its entries: chunks of 8
+};
+
+// First cell of tile 0 along x: the padded tile then starts at an even grid
+// point, which bulk copies of single 8-byte points need (16-byte starts).
+__host__ __device__ inline int tile_shift(const Geom &g) { return g.Ra[0] & 1; }
+// z cells of a slab and slabs of a tile
+inline int slab_cells(const Geom &g) { return g.is2d ? 1 : 2; }
+inline int slabs_per_tile(const Geom &g) { return g.is2d ? 1 : g.T[2] / 2; }
+
 // Slots of a plan's small device work buffer (int[16]).
 constexpr int kWorkGather = 0;   // work counter of the persistent gather
 constexpr int kWorkSpread = 1;   // work counter of the persistent spread
 constexpr int kWorkTapFill = 2;  // stored-H build: fill disagrees with count
 constexpr int kWorkStatus = 3;   // interpolation status (a bounded wait expired)
+constexpr int kWorkGatherTab = 4;  // [2] stored-H gather: next chunk, blocks done (the last one clears both)
 constexpr int kDefaultWaitPolls = 1 << 22;
 
 struct BatchInterp {
@@ -198,8 +216,6 @@ struct BatchInterp {
     int tmap_ok;               // bit log2(width): that map is valid
     int nc;
     float scale;
-    const uint32_t *tap_rows;  // the volume's stored H (8-coil gather entries), or null
-    const int2 *tap_ent;
     InterpStatus status;       // the volume's plan: its status flag and wait polls
 };
 
@@ -233,10 +249,8 @@ struct BatchFFTParams {
 
 int batch_four_step(int K, bool all_vec16);
 int launch_fft_batch_p(const BatchFFTParams &P, int kind, size_t smem, bool rare, int r1, cudaStream_t s);
-// stored_h: every volume has its stored H (the 8-coil gather group then reads it)
 int launch_interp_batch(bool gather, int cb, int R, bool radial, const BatchInterp *vols, const int4 *table,
-                        int nblocks, size_t smem, const KBParams &kb, int *work, int nsm, cudaStream_t s,
-                        bool stored_h);
+                        int nblocks, size_t smem, const KBParams &kb, int *work, int nsm, cudaStream_t s);
 int launch_perm_batch(bool out, const BatchPerm *vols, const int4 *table, int nblocks, cudaStream_t s);
 
 // ----------------------------------------------------------------- plan
@@ -315,6 +329,7 @@ struct nufft3d_plan {
     nufft3d::Cand cand_desc{};         // device list + per-sub-cube starts and lengths
     int64_t n_blocks = 0;
     std::vector<int32_t> tile_counts;  // in-bounds samples per tile (host copy; pieces are rebuilt from it)
+    std::vector<int32_t> slab_counts;  // the same per slab, while the plan is built
     int piece_samples = 0;      // largest piece (samples) of the current piece table
     int coils_per_pass = 8;
     int max_coils_per_pass = 8; // the largest coil width the plan's shared memory allows
@@ -326,11 +341,14 @@ struct nufft3d_plan {
     int *work = nullptr;        // [16]: work counters of the persistent interpolation kernels and the
                                 // plan's status flags (slots kWork*)
     int wait_polls = nufft3d::kDefaultWaitPolls;  // polls of each bounded wait in the gather
-    // stored H in tile order (8-coil passes): row of sorted sample s = entries
-    // [8*tap_rows[s], 8*tap_rows[s+1]) of tap_ent, (weight bits, tile offset),
-    // padded with zero weights to whole chunks of 8
-    uint32_t *tap_rows = nullptr;
-    int2 *tap_ent = nullptr;
+    // stored H (gather_tab.cu): records, ranges of records, first chunk of each
+    // row of four samples, weights and points of the entries
+    nufft3d::GatherRec *grecs = nullptr;
+    int2 *gchunks = nullptr;
+    int n_gchunks = 0;
+    uint32_t *grow = nullptr;
+    float4 *gw = nullptr;
+    uint32_t *gi = nullptr;
     int64_t tap_bytes = 0;
     // stored H' for the 8-coil spread (tables.cu): pieces of at most
     // kSpreadCap samples, (tile, first sample, count, first line); the warps'
@@ -384,12 +402,20 @@ int launch_gather(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, float sc
                   const float *wsample, cudaStream_t s);
 // plan time: per-block bound on summed weights (blocks[b].w) for the spread
 int launch_weight_sum(nufft3d_plan *p, cudaStream_t s);
-// plan time, stored H: rows[s] = chunks of 8 entries in sample s's row
+// plan time, entries for the build of the stored H': rows[s] = chunks of 8
+// entries in sample s's row, then the entries (rows = chunk offsets)
 int launch_tap_count(nufft3d_plan *p, uint32_t *rows, cudaStream_t s);
-// plan time, stored H: the entries of every row (rows = chunk offsets)
 int launch_tap_fill(nufft3d_plan *p, const uint32_t *rows, int2 *taps, cudaStream_t s);
-// the stored-H kernels serve this plan (8-coil passes, R <= 3)
+// the stored tables serve this plan (8-coil passes, R <= 3)
 bool tap_table_applies(const nufft3d_plan *p);
+// stored H (gather_tab.cu): plan-time build, and the gather of coils
+// c0..c0+cb-1 that reads it (cb 1, 2, 4 or 8)
+int build_gather_table(nufft3d_plan *p, int mode, cudaStream_t s);
+int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int c0, int cb, float scale,
+                      const float *ws, cudaStream_t s);
+int configure_gather_tab_kernels();
+// the map of the grid for bulk copies of one plane of a padded tile, cb coils
+bool encode_plane_map(const nufft3d_plan *p, const float2 *G, int nc, int cb, CUtensorMap *m);
 // spread: G += H' ks (G zeroed by caller)
 int launch_spread(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, cudaStream_t s);
 // Largest spread piece of the stored H' (samples staged in shared memory,
@@ -397,7 +423,7 @@ int launch_spread(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, cudaStre
 constexpr int kSpreadCap = 1664;
 // stored H' (tables.cu): plan-time build from the stored H, the 8-coil
 // spread pass that reads it, and whether it serves coils c0..c0+7 of nc
-int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s);
+int build_spread_table(nufft3d_plan *p, int mode, const uint32_t *rows, const int2 *taps, cudaStream_t s);
 int launch_spread_tab(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, int c0, cudaStream_t s);
 bool spread_tab_applies(const nufft3d_plan *p, int nc, int c0);
 int configure_spread_tab_kernels();

@@ -27,6 +27,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "async.h"
 #include "internal.h"
 
 namespace nufft3d {
@@ -378,62 +379,19 @@ __device__ __forceinline__ int eval_pair(int base, const SampleGeo &sg, const Ca
 // the host-pointer entry points), lets the copy land with a second bounded
 // wait and returns.
 
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity)
-{
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(bar), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ void tma_load_4d(unsigned dst, const CUtensorMap *map, int c0, int c1, int c2, int c3,
-                                            unsigned bar)
-{
-    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                 " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-                 : "memory");
-}
-
 // Origin of the padded tile of tile index tid; true if it lies inside the
 // grid on every axis (no wrap-around).
 __device__ __forceinline__ bool tile_origin(const Geom &g, int tid, int &ox, int &oy, int &oz)
 {
-    const int tx = tid % g.nt[0];
-    const int ty = (tid / g.nt[0]) % g.nt[1];
-    const int tz = tid / (g.nt[0] * g.nt[1]);
-    ox = tx * g.T[0] - g.Ra[0];
+    const int tz = tid % g.nt[2];  // z fastest: the tiles of a column are neighbours
+    const int tx = (tid / g.nt[2]) % g.nt[0];
+    const int ty = tid / (g.nt[2] * g.nt[0]);
+    ox = tx * g.T[0] + tile_shift(g) - g.Ra[0];
     oy = ty * g.T[1] - g.Ra[1];
     oz = tz * g.T[2] - g.Ra[2];
     return ox >= 0 && oy >= 0 && oz >= 0 && ox + g.P[0] <= g.K[0] && oy + g.P[1] <= g.K[1] &&
            oz + g.P[2] <= g.K[2];
 }
-
-// Bounded wait for the phase of the given parity (at most `polls` polls);
-// false if it expired.
-constexpr int kDrainPolls = 1 << 22;
-
-__device__ __forceinline__ bool mbar_wait_bounded(unsigned bar, unsigned parity, int polls)
-{
-    for (int i = 0; i < polls; ++i)
-        if (mbar_try_wait(bar, parity)) return true;
-    return false;
-}
-
 
 __device__ __forceinline__ float2 *align128(float4 *p)
 {
@@ -943,167 +901,7 @@ k_weight_sum(const float4 *__restrict__ samples, int4 *__restrict__ blocks, Geom
     if (threadIdx.x == 0) blocks[blockIdx.x].w = __float_as_int(m * 1.001f + 1e-3f);
 }
 
-// ------------------------------------------------------------- stored H
-// The reference keeps H as a sparse matrix (nufft_3d.m:153-212).  Its stored
-// form here follows the tile sort: the row of sorted sample s is a run of
-// (weight bits, tile offset) entries in chunks of 8 taps, padded with zero
-// weights to a whole chunk; the rows of a piece are contiguous, so the gather
-// streams them with plain loads that run ahead of the taps and evaluates no
-// kernel weights.  Inside a row the taps are ordered for the shared-memory
-// banks: round-robin over the residue of the tile offset mod 8, and inside
-// each chunk even offsets before odd ones (gather lanes k and k+4 read one
-// 16-byte column of the point-major tile, conflict-free when their offsets
-// differ in parity: about 0.12 collisions per chunk on J=6 radial rows).
-// The residue order would also keep a chunk's 8 taps on distinct banks of
-// the spread's integer planes (about 1.13 wavefronts per chunk), but a
-// spread that streams H through shared memory measured slower than one that
-// evaluates the kernel (staging H costs as many instructions as the weights
-// it saves), so H' is applied on the fly.  The weights are the on-the-fly
-// kernels' (same candidate lists and kernel).
-
-// Streaming load of one stored-H entry (read once: no L1 allocation).
-__device__ __forceinline__ int2 ld_tap(const int2 *p)
-{
-    int2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
-
-// One tile piece of the gather from the stored H (8 coils per pass).  Each
-// group of 8 lanes takes a contiguous run of the piece's samples, whose rows
-// form one contiguous stream of chunks; lane l of the group applies entry l
-// of every chunk (a whole tap: 8 coils, rotated coil-pair reads as in the
-// on-the-fly gather) and keeps the next 4 chunks' entries in registers, so
-// the loads run ahead across sample boundaries (2, 3 or 6 chunks in
-// registers, a 5-deep per-lane shared-memory FIFO filled by asynchronous
-// copies, and L2 prefetch windows all measured slower).  At the end of a
-// sample the group reduces its 8 partial sums.
-template <int R>
-__device__ __forceinline__ bool gather_piece_tab(const float2 *__restrict__ G, float2 *__restrict__ ks, int nc,
-                                                 int c0, const int4 bi, const Geom &g, float scale,
-                                                 const float *__restrict__ wsample,
-                                                 const uint32_t *__restrict__ rows, const int2 *__restrict__ taps,
-                                                 float2 *tile, const CUtensorMap *tmap, unsigned bar_sa,
-                                                 unsigned &phase, const InterpStatus &stat)
-{
-    constexpr int CB = 8;
-    const int lane = threadIdx.x & 31, lig = lane & 7;
-    const int grp = threadIdx.x >> 3, ngrp = blockDim.x >> 3;
-    const unsigned gmask = 0xFFu << (lane & 24);
-    const int s_lo = bi.y + (int)(((long long)bi.z * grp) / ngrp);
-    const int s_hi = bi.y + (int)(((long long)bi.z * (grp + 1)) / ngrp);
-    uint32_t cA = 0, nchk = 0;
-    if (s_lo < s_hi) {
-        cA = __ldg(&rows[s_lo]);
-        nchk = __ldg(&rows[s_hi]) - cA;
-    }
-    const int2 *st = taps + (size_t)cA * 8 + lig;
-    const int2 z2 = make_int2(0, 0);
-    // the first chunks land while the tile does
-    int2 e0 = nchk > 0 ? ld_tap(st) : z2;
-    int2 e1 = nchk > 1 ? ld_tap(st + 8) : z2;
-    int2 e2 = nchk > 2 ? ld_tap(st + 16) : z2;
-    int2 e3 = nchk > 3 ? ld_tap(st + 24) : z2;
-    if (!stage_tile<CB>(G, nc, c0, bi, g, tile, tmap, bar_sa, phase, stat)) return false;
-    const int cb = min(CB, nc - c0);
-    const int rot = lig & 3, rot16 = rot << 4;
-    float2 acc[CB];
-#pragma unroll
-    for (int c = 0; c < CB; ++c) acc[c] = make_float2(0.f, 0.f);
-    int s = s_lo;
-    uint32_t send = s < s_hi ? __ldg(&rows[s + 1]) - cA : 0u;      // chunk where sample s ends
-    uint32_t snext = s + 1 < s_hi ? __ldg(&rows[s + 2]) - cA : 0u;  // and sample s+1
-    // write sample s, move to the next one.  Reduce-scatter over the group:
-    // at each of 3 steps a lane keeps half of its coils (the half named by
-    // one bit of its lane index) and adds the partner's copy of them, so lane
-    // l ends with coil l summed over the 8 lanes (14 shuffles instead of 48).
-    auto finish = [&]() {
-        unrotate<CB>(acc, rot);
-        float2 h4[4], h2[2], h1;
-        const bool b2 = lig & 4, b1 = lig & 2, b0 = lig & 1;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float2 keep = b2 ? acc[4 + k] : acc[k], give = b2 ? acc[k] : acc[4 + k];
-            h4[k].x = keep.x + __shfl_xor_sync(gmask, give.x, 4);
-            h4[k].y = keep.y + __shfl_xor_sync(gmask, give.y, 4);
-        }
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const float2 keep = b1 ? h4[2 + k] : h4[k], give = b1 ? h4[k] : h4[2 + k];
-            h2[k].x = keep.x + __shfl_xor_sync(gmask, give.x, 2);
-            h2[k].y = keep.y + __shfl_xor_sync(gmask, give.y, 2);
-        }
-        {
-            const float2 keep = b0 ? h2[1] : h2[0], give = b0 ? h2[0] : h2[1];
-            h1.x = keep.x + __shfl_xor_sync(gmask, give.x, 1);
-            h1.y = keep.y + __shfl_xor_sync(gmask, give.y, 1);
-        }
-        const float sc_ = wsample ? scale * __ldg(&wsample[s]) : scale;
-        if (lig < cb) ks[(size_t)s * nc + c0 + lig] = make_float2(h1.x * sc_, h1.y * sc_);
-#pragma unroll
-        for (int c = 0; c < CB; ++c) acc[c] = make_float2(0.f, 0.f);
-        ++s;
-        send = snext;
-        snext = s + 1 < s_hi ? __ldg(&rows[s + 2]) - cA : 0u;
-    };
-    while (s < s_hi && send == 0u) finish();  // samples without taps
-    auto step = [&](int2 &ed, uint32_t ch) {
-        const int2 cur = ed;
-        ed = ch + 4 < nchk ? ld_tap(st + (size_t)(ch + 4) * 8) : z2;
-        // coil pairs in the rotated order rot ^ k (see accumulate); padding
-        // entries (weight 0, tile offset 0) add nothing and need no branch
-        const float w = __int_as_float(cur.x);
-        const float2 ww = make_float2(w, w);
-        const char *pb = reinterpret_cast<const char *>(tile) + (size_t)cur.y * (CB * 8);
-#pragma unroll
-        for (int k = 0; k < CB / 2; ++k) {
-            const float4 v = *reinterpret_cast<const float4 *>(pb + (rot16 ^ (k << 4)));
-            acc[2 * k] = __ffma2_rn(ww, make_float2(v.x, v.y), acc[2 * k]);
-            acc[2 * k + 1] = __ffma2_rn(ww, make_float2(v.z, v.w), acc[2 * k + 1]);
-        }
-        if (ch + 1 == send) {
-            do {
-                finish();
-            } while (s < s_hi && send == ch + 1);  // and the samples without taps after it
-        }
-    };
-    for (uint32_t ch = 0; ch < nchk; ch += 4) {
-        step(e0, ch);
-        if (ch + 1 < nchk) step(e1, ch + 1);
-        if (ch + 2 < nchk) step(e2, ch + 2);
-        if (ch + 3 < nchk) step(e3, ch + 3);
-    }
-    __syncthreads();  // every warp is done with the tile
-    return true;
-}
-
-// Persistent gather from the stored H: shared memory = the tile.
-template <int R>
-__global__ void __launch_bounds__(kInterpThreads)
-k_gather_tab(const float2 *__restrict__ G, float2 *__restrict__ ks, int nc, int c0,
-             const int4 *__restrict__ blocks, int nblocks, int *__restrict__ work, Geom g, float scale,
-             const float *__restrict__ wsample, const uint32_t *__restrict__ rows, const int2 *__restrict__ taps,
-             const __grid_constant__ CUtensorMap tmap, int use_tma, InterpStatus st)
-{
-    extern __shared__ float4 smem4[];
-    __shared__ unsigned long long bar;
-    __shared__ int next;
-    float2 *tile = align128(smem4);
-    const unsigned bar_sa = (unsigned)__cvta_generic_to_shared(&bar);
-    if (threadIdx.x == 0) mbar_init(bar_sa, 1);
-    __syncthreads();
-    unsigned phase = 0;
-    for (;;) {
-        if (threadIdx.x == 0) next = atomicAdd(work, 1);
-        __syncthreads();
-        const int b = next;
-        if (b >= nblocks) break;
-        if (!gather_piece_tab<R>(G, ks, nc, c0, blocks[b], g, scale, wsample, rows, taps, tile,
-                                 use_tma ? &tmap : nullptr, bar_sa, phase, st))
-            return;
-    }
-}
-
+// ------------------------------------------- entries for the stored H' build
 // Weight and tile offset of candidate ci for the stored H.  The distance is
 // formed with explicitly rounded operations (never contracted into FMAs), so
 // the count and fill passes, compiled separately, take identical support
@@ -1323,36 +1121,6 @@ k_gather_batch(const BatchInterp *__restrict__ vols, const int4 *__restrict__ ta
     }
 }
 
-// Batched 8-coil gather when every volume has its stored H: the table entry
-// (volume, piece, first coil) selects the volume's rows; shared memory = the
-// tile only.
-template <int R>
-__global__ void __launch_bounds__(kInterpThreads)
-k_gather_batch_tab(const BatchInterp *__restrict__ vols, const int4 *__restrict__ table, int ntab,
-                   int *__restrict__ work)
-{
-    extern __shared__ float4 smem4[];
-    __shared__ unsigned long long bar;
-    __shared__ int next;
-    float2 *tile = align128(smem4);
-    const unsigned bar_sa = (unsigned)__cvta_generic_to_shared(&bar);
-    if (threadIdx.x == 0) mbar_init(bar_sa, 1);
-    __syncthreads();
-    unsigned phase = 0;
-    for (;;) {
-        if (threadIdx.x == 0) next = atomicAdd(work, 1);
-        __syncthreads();
-        const int t = next;
-        if (t >= ntab) break;
-        const int4 e = table[t];
-        const BatchInterp &b = vols[e.x];
-        const CUtensorMap *tm = (b.tmap_ok >> 3) & 1 ? &b.tmaps[3] : nullptr;
-        if (!gather_piece_tab<R>(b.in, b.out, b.nc, e.z, b.blocks[e.y], b.g, b.scale, b.wsample, b.tap_rows,
-                                 b.tap_ent, tile, tm, bar_sa, phase, b.status))
-            return;
-    }
-}
-
 template <int CB, bool RADIAL, int R>
 __global__ void __launch_bounds__(kInterpThreads)
 k_spread_batch(const BatchInterp *__restrict__ vols, const int4 *__restrict__ table, int ntab,
@@ -1447,8 +1215,7 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 // coils per point); false where it does not apply (odd nc: row strides must
 // be multiples of 16 bytes; single coils: the box row must be 16 bytes or
 // more) or the driver refuses it.
-template <int CB>
-static bool gather_tensor_map(const nufft3d_plan *p, const float2 *G, int nc, CUtensorMap *m)
+static bool grid_box_map(const nufft3d_plan *p, const float2 *G, int nc, int CB, int Pz, CUtensorMap *m)
 {
     const Geom &g = p->geom;
     if (CB < 2 || nc % 2) return false;
@@ -1457,23 +1224,45 @@ static bool gather_tensor_map(const nufft3d_plan *p, const float2 *G, int nc, CU
     const cuuint64_t row = (cuuint64_t)nc * sizeof(float2);
     cuuint64_t dim[4] = {(cuuint64_t)2 * nc, (cuuint64_t)g.K[0], (cuuint64_t)g.K[1], (cuuint64_t)g.K[2]};
     cuuint64_t str[3] = {row, row * g.K[0], row * g.K[0] * g.K[1]};
-    cuuint32_t box[4] = {2 * CB, (cuuint32_t)g.P[0], (cuuint32_t)g.P[1], (cuuint32_t)g.P[2]};
+    cuuint32_t box[4] = {(cuuint32_t)(2 * CB), (cuuint32_t)g.P[0], (cuuint32_t)g.P[1], (cuuint32_t)Pz};
     cuuint32_t es[4] = {1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float2 *>(G), dim, str, box, es,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+template <int CB>
+static bool gather_tensor_map(const nufft3d_plan *p, const float2 *G, int nc, CUtensorMap *m)
+{
+    return grid_box_map(p, G, nc, CB, p->geom.P[2], m);
+}
+
 // Encodes the gather tensor map of grid G (nc coils) for chunks of cb
 // coils; false where the bulk copy does not apply.
 bool encode_gather_map(const nufft3d_plan *p, const float2 *G, int nc, int cb, CUtensorMap *m)
 {
-    switch (cb) {
-    case 2: return gather_tensor_map<2>(p, G, nc, m);
-    case 4: return gather_tensor_map<4>(p, G, nc, m);
-    case 8: return gather_tensor_map<8>(p, G, nc, m);
-    default: return false;
-    }
+    return grid_box_map(p, G, nc, cb, p->geom.P[2], m);
+}
+
+bool encode_plane_map(const nufft3d_plan *p, const float2 *G, int nc, int cb, CUtensorMap *m)
+{
+    if (cb % 2 == 0) return grid_box_map(p, G, nc, cb, 1, m);
+    // an odd coil count in one pass: a 3-D map of rows of points with all
+    // their coils (rows of K1 points, K1 even, and boxes of P0 points, P0 and
+    // their first point even, are whole 16-byte units)
+    const Geom &g = p->geom;
+    const cuuint32_t inner = (cuuint32_t)(2 * nc * g.P[0]);
+    if (cb != nc || inner > 256 || g.K[0] % 2) return false;
+    auto enc = tensor_map_encoder();
+    if (!enc) return false;
+    const cuuint64_t row = (cuuint64_t)nc * g.K[0] * sizeof(float2);
+    cuuint64_t dim[3] = {(cuuint64_t)2 * nc * g.K[0], (cuuint64_t)g.K[1], (cuuint64_t)g.K[2]};
+    cuuint64_t str[2] = {row, row * g.K[1]};
+    cuuint32_t box[3] = {inner, (cuuint32_t)g.P[1], 1};
+    cuuint32_t es[3] = {1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float2 *>(G), dim, str, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 int plan_check_status(nufft3d_plan *p, cudaStream_t s)
@@ -1528,35 +1317,6 @@ int interp_grid_sms(const nufft3d_plan *p)
 
 bool tap_table_applies(const nufft3d_plan *p) { return p->coils_per_pass == 8 && p->geom.R <= 3; }
 
-template <int R>
-static int gather_tab_t(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int c0, float scale,
-                        const float *ws, cudaStream_t s)
-{
-    const size_t smem = smem_plane_bytes(R, 8) + 128;
-    alignas(64) CUtensorMap m;
-    std::memset(&m, 0, sizeof(m));
-    const int use_tma = p->use_tma && gather_tensor_map<8>(p, G, nc, &m) ? 1 : 0;
-    NUFFT_CUDA_TRY(cudaMemsetAsync(p->work, 0, sizeof(int), s));
-    const int64_t grid = std::min<int64_t>(p->n_blocks, interp_grid_sms(p));
-    k_gather_tab<R><<<(unsigned)grid, kInterpThreads, smem, s>>>(G, ks, nc, c0, p->blocks, (int)p->n_blocks,
-                                                                 p->work, p->geom, scale, ws, p->tap_rows,
-                                                                 p->tap_ent, m, use_tma, plan_status(p));
-    NUFFT_CUDA_TRY(cudaGetLastError());
-    return NUFFT3D_SUCCESS;
-}
-
-// 8-coil gather passes of a plan with the stored H
-static int gather_tab(nufft3d_plan *p, const float2 *in, float2 *out, int nc, int c0, float scale,
-                      const float *ws, cudaStream_t s)
-{
-    switch (p->geom.R) {
-    case 1: return gather_tab_t<1>(p, in, out, nc, c0, scale, ws, s);
-    case 2: return gather_tab_t<2>(p, in, out, nc, c0, scale, ws, s);
-    case 3: return gather_tab_t<3>(p, in, out, nc, c0, scale, ws, s);
-    default: return fail(NUFFT3D_ERR_UNSUPPORTED, "stored H with R > 3");
-    }
-}
-
 template <bool GATHER, int CB, bool RADIAL>
 static int dispatch_r(nufft3d_plan *p, const float2 *in, float2 *out, int nc, int c0, float scale,
                       const float *ws, cudaStream_t s)
@@ -1594,16 +1354,18 @@ static int interp(nufft3d_plan *p, const float2 *in, float2 *out, int nc, float 
         int cb = 1;
         while (cb < rem && cb < cmax) cb *= 2;
         int st;
+        if (GATHER && p->gw) {  // the stored H, any coil width
+            NUFFT_TRY(launch_gather_tab(p, in, out, nc, c0, cb, scale, ws, s));
+            if (cb > rem) break;
+            continue;
+        }
         switch (cb) {
         case 1: st = dispatch<GATHER, 1>(p, in, out, nc, c0, scale, ws, s); break;
         case 2: st = dispatch<GATHER, 2>(p, in, out, nc, c0, scale, ws, s); break;
         case 4: st = dispatch<GATHER, 4>(p, in, out, nc, c0, scale, ws, s); break;
         default:
-            // the stored H serves the gather and the stored H' the spread
-            // (full passes of an even coil count), else the kernel is evaluated
-            if (GATHER && p->tap_ent)
-                st = gather_tab(p, in, out, nc, c0, scale, ws, s);
-            else if (!GATHER && spread_tab_applies(p, nc, c0))
+            // the stored H' serves the spread of full passes of an even coil count
+            if (!GATHER && spread_tab_applies(p, nc, c0))
                 st = launch_spread_tab(p, in, out, nc, c0, s);
             else
                 st = dispatch<GATHER, 8>(p, in, out, nc, c0, scale, ws, s);
@@ -1725,22 +1487,9 @@ static int interp_batch_r(bool gather, int R, const BatchInterp *vols, const int
 }
 
 int launch_interp_batch(bool gather, int cb, int R, bool radial, const BatchInterp *vols, const int4 *table,
-                        int nblocks, size_t smem, const KBParams &kb, int *work, int nsm, cudaStream_t s,
-                        bool stored_h)
+                        int nblocks, size_t smem, const KBParams &kb, int *work, int nsm, cudaStream_t s)
 {
     if (nblocks <= 0) return NUFFT3D_SUCCESS;
-    if (gather && cb >= 8 && stored_h && R <= 3) {
-        NUFFT_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(int), s));
-        const int grid = nblocks < nsm ? nblocks : nsm;
-        const size_t sm = smem_plane_bytes(R, 8) + 128;
-        switch (R) {
-        case 1: k_gather_batch_tab<1><<<grid, kInterpThreads, sm, s>>>(vols, table, nblocks, work); break;
-        case 2: k_gather_batch_tab<2><<<grid, kInterpThreads, sm, s>>>(vols, table, nblocks, work); break;
-        default: k_gather_batch_tab<3><<<grid, kInterpThreads, sm, s>>>(vols, table, nblocks, work); break;
-        }
-        NUFFT_CUDA_TRY(cudaGetLastError());
-        return NUFFT3D_SUCCESS;
-    }
     if (cb >= 8) return radial ? interp_batch_r<8, true>(gather, R, vols, table, nblocks, smem, kb, work, nsm, s)
                                : interp_batch_r<8, false>(gather, R, vols, table, nblocks, smem, kb, work, nsm, s);
     if (cb >= 4) return radial ? interp_batch_r<4, true>(gather, R, vols, table, nblocks, smem, kb, work, nsm, s)
@@ -1806,12 +1555,6 @@ int configure_interp_kernels()
     NUFFT_TRY(allow_smem(k_tap_count<false>));
     NUFFT_TRY(allow_smem(k_tap_fill<true>));
     NUFFT_TRY(allow_smem(k_tap_fill<false>));
-    NUFFT_TRY(allow_smem(k_gather_batch_tab<1>));
-    NUFFT_TRY(allow_smem(k_gather_batch_tab<2>));
-    NUFFT_TRY(allow_smem(k_gather_batch_tab<3>));
-    NUFFT_TRY(allow_smem(k_gather_tab<1>));
-    NUFFT_TRY(allow_smem(k_gather_tab<2>));
-    NUFFT_TRY(allow_smem(k_gather_tab<3>));
     NUFFT_TRY(cfg_cb<1>());
     NUFFT_TRY(cfg_cb<2>());
     NUFFT_TRY(cfg_cb<4>());

@@ -284,7 +284,9 @@ static const CandSet &candidate_set(int R, int radial, int is2d, double J, int P
 struct KeyParams {
     double u;
     int K[3], T[3], nt[3], Ra[3];
+    int shift[3];  // first cell of tile 0
     int is2d;
+    int slab_cells, slabs;  // z cells of a slab, slabs of a tile
     uint32_t ntiles;
 };
 
@@ -294,9 +296,58 @@ __device__ __forceinline__ int64_t wrap64(int64_t x, int64_t K)
     return r < 0 ? r + K : r;
 }
 
-// nufft_3d.m:120-125: om scaled by u in double; ok mask; tile key.
+// Grid index of oversampled frequency x: the grid is stored with frequency 0
+// in its middle (index K/2; K is even, or 1 along z in 2-D), so that the
+// padded tiles that wrap around the grid edge, which cost more to stage, hold
+// the sparse rim of k-space and not its dense centre.  The shift by K/2 is a
+// factor (-1)^n per axis on the image side, carried by the signs of U.
+__device__ __forceinline__ int64_t grid_index(int64_t x, int64_t K) { return wrap64(x + K / 2, K); }
+
+// Position of (x, y, z) along a Hilbert curve through a cube of 2^B points a
+// side (square for D = 2), by Skilling's transposed form (AIP Conf. Proc. 707,
+// 381, 2004): Gray-code the coordinates from the top bit down, undoing the
+// rotation of each level, then interleave the bits.
+template <int D, int B>
+__device__ __forceinline__ uint32_t hilbert_index(uint32_t (&X)[3])
+{
+#pragma unroll
+    for (uint32_t q = 1u << (B - 1); q > 1; q >>= 1) {
+        const uint32_t low = q - 1;
+#pragma unroll
+        for (int i = 0; i < D; ++i) {
+            if (X[i] & q) {
+                X[0] ^= low;
+            } else {
+                const uint32_t t = (X[0] ^ X[i]) & low;
+                X[0] ^= t;
+                X[i] ^= t;
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 1; i < D; ++i) X[i] ^= X[i - 1];
+    uint32_t t = 0;
+#pragma unroll
+    for (uint32_t q = 1u << (B - 1); q > 1; q >>= 1)
+        if (X[D - 1] & q) t ^= q - 1;
+    uint32_t h = 0;
+#pragma unroll
+    for (int b = B - 1; b >= 0; --b)
+#pragma unroll
+        for (int i = 0; i < D; ++i) h = (h << 1) | (((X[i] ^ t) >> b) & 1u);
+    return h;
+}
+
+// nufft_3d.m:120-125: om scaled by u in double; ok mask; sort key: the tile (z
+// fastest, so that the tiles of a column are neighbours), its slab, and the
+// position along a Hilbert curve at half-cell resolution inside the tile's
+// slab (the stored tables take consecutive samples together: on the 128^3
+// koosh ball four consecutive samples reach 172 grid points between them,
+// against 180 in Morton order).
+constexpr int kCurveBits = 12;
+
 __global__ void k_keys(const double *__restrict__ om, int64_t M, KeyParams kp,
-                       uint32_t *__restrict__ keys, int32_t *__restrict__ vals)
+                       uint64_t *__restrict__ keys, int32_t *__restrict__ vals)
 {
     const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
@@ -307,26 +358,39 @@ __global__ void k_keys(const double *__restrict__ om, int64_t M, KeyParams kp,
         ok = ok && og[a] >= -kp.K[a] / 2.0 && og[a] <= kp.K[a] / 2.0 - 1;
     }
     if (kp.is2d) ok = true; // nufft_3d.m:125 ('... & ok | N(3)==1')
-    uint32_t key = kp.ntiles;
+    uint64_t key = (uint64_t)kp.ntiles * kp.slabs << kCurveBits;
     if (ok) {
-        int t[3];
+        int t[3], l[3];
+        uint32_t half[3];  // position inside the tile in half cells
         for (int a = 0; a < 3; ++a) {
-            const int64_t b = wrap64((int64_t)round(og[a]), kp.K[a]);
+            const double r = round(og[a]);
+            const int64_t b = grid_index((int64_t)r - kp.shift[a], kp.K[a]);
             t[a] = (int)(b / kp.T[a]);
+            l[a] = (int)(b - (int64_t)t[a] * kp.T[a]);
+            half[a] = 2u * (uint32_t)l[a] + (og[a] >= r ? 1u : 0u);
         }
-        key = (uint32_t)(t[0] + kp.nt[0] * (t[1] + kp.nt[1] * t[2]));
+        const uint64_t tile = (uint64_t)t[2] + (uint64_t)kp.nt[2] * ((uint64_t)t[0] + (uint64_t)kp.nt[0] * t[1]);
+        uint32_t slab = 0, h;
+        if (kp.is2d) {
+            h = hilbert_index<2, 6>(half);
+        } else {
+            slab = (uint32_t)(l[2] / kp.slab_cells);
+            half[2] &= (uint32_t)(2 * kp.slab_cells - 1);
+            h = hilbert_index<3, 4>(half);
+        }
+        key = ((tile * kp.slabs + slab) << kCurveBits) | h;
     }
     keys[m] = key;
     vals[m] = (int32_t)m;
 }
 
-__global__ void k_hist(const uint32_t *__restrict__ keys, int64_t M, uint32_t ntiles,
+__global__ void k_hist(const uint64_t *__restrict__ keys, int64_t M, uint32_t nslabs,
                        int32_t *__restrict__ counts)
 {
     const int64_t m = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
-    const uint32_t k = keys[m];
-    if (k < ntiles) atomicAdd(&counts[k], 1);
+    const uint64_t k = keys[m] >> kCurveBits;
+    if (k < nslabs) atomicAdd(&counts[k], 1);
 }
 
 __global__ void k_records(const double *__restrict__ om, const int32_t *__restrict__ perm,
@@ -342,7 +406,7 @@ __global__ void k_records(const double *__restrict__ om, const int32_t *__restri
         const double og = kp.u * om[3 * (int64_t)m + a];
         const double r = round(og);
         f[a] = (float)(og - r);
-        const int64_t b = wrap64((int64_t)r, kp.K[a]);
+        const int64_t b = grid_index((int64_t)r - kp.shift[a], kp.K[a]);
         const int64_t t = b / kp.T[a];
         l[a] = (int)(b - t * kp.T[a]) + kp.Ra[a];
     }
@@ -403,6 +467,7 @@ int configure_kernels()
     NUFFT_DEVICE_LOCK; // constant-memory uploads must not overlap a stream capture
     NUFFT_TRY(configure_fft_kernels());
     NUFFT_TRY(configure_interp_kernels());
+    NUFFT_TRY(configure_gather_tab_kernels());
     NUFFT_TRY(configure_spread_tab_kernels());
     if (dev < 32) done_mask |= 1 << dev;
     return NUFFT3D_SUCCESS;
@@ -425,7 +490,7 @@ static void adopt_tables(nufft3d_plan *p)
     auto t = std::make_shared<TableOwner>();
     t->device = p->device;
     t->ptrs = {p->samples, p->perm, p->inv, p->blocks, p->cand, p->U, p->d, p->d_orig,
-               p->tw[0], p->tw[1], p->tw[2], p->tap_rows, p->tap_ent, p->spread_pieces, p->spread_wstart, p->spread_ent};
+               p->tw[0], p->tw[1], p->tw[2], p->grecs, p->gchunks, p->grow, p->gw, p->gi, p->spread_pieces, p->spread_wstart, p->spread_ent};
     p->tables = t;
 }
 
@@ -446,8 +511,11 @@ static void free_plan_memory(nufft3d_plan *p)
         F(p->d);
         F(p->d_orig);
         for (int a = 0; a < 3; ++a) F(p->tw[a]);
-        F(p->tap_rows);
-        F(p->tap_ent);
+        F(p->grecs);
+        F(p->gchunks);
+        F(p->grow);
+        F(p->gw);
+        F(p->gi);
         F(p->spread_pieces);
         F(p->spread_wstart);
         F(p->spread_ent);
@@ -496,18 +564,19 @@ static int dmalloc(T **ptr, size_t count, int64_t *acc)
     return NUFFT3D_SUCCESS;
 }
 
-// The stored H (nufft_3d.m:153-212) in tile order: count each row's chunks,
-// scan them into row offsets, then fill the rows.  mode 0 = none, 1 = always,
-// -1 = when it takes at most half of the free device memory.
-static int build_tap_table(nufft3d_plan *p, int mode, std::vector<void *> &tmp, cudaStream_t s)
+// The taps of every sample in tile order, (weight bits, tile offset) in rows
+// padded to whole chunks of 8, from which the stored H' is built: count each
+// row's chunks, scan them into row offsets, then fill the rows.  *ent stays
+// null where the memory does not suffice and mode allows to do without.
+static int build_taps(nufft3d_plan *p, int mode, std::vector<void *> &tmp, uint32_t **rows_out, int2 **ent,
+                      cudaStream_t s)
 {
-    if (mode == 0 || p->nnz == 0 || !tap_table_applies(p)) return NUFFT3D_SUCCESS;
     const int64_t nnz = p->nnz;
     int maxcnt = 0;
     for (int q = 0; q < 8; ++q) maxcnt = std::max(maxcnt, p->cand_desc.cnt[q]);
     if ((uint64_t)nnz * (uint64_t)((maxcnt + 7) / 8) >= 0xffffffffull) {  // row offsets are 32-bit chunk indices
         if (mode < 0) return NUFFT3D_SUCCESS;
-        return fail(NUFFT3D_ERR_SIZE, "too many samples for the stored H");
+        return fail(NUFFT3D_ERR_SIZE, "too many samples for the stored H'");
     }
     uint32_t *cnt = nullptr;
     NUFFT_TRY(dmalloc(&cnt, (size_t)nnz + 1, nullptr));
@@ -521,40 +590,23 @@ static int build_tap_table(nufft3d_plan *p, int mode, std::vector<void *> &tmp, 
     tmp.push_back(tstore);
     uint32_t *rows = nullptr;
     NUFFT_TRY(dmalloc(&rows, (size_t)nnz + 1, nullptr));
+    tmp.push_back(rows);
     uint32_t total = 0;
-    cudaError_t e = cub::DeviceScan::ExclusiveSum(tstore, tb, cnt, rows, (int)(nnz + 1), s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&total, rows + nnz, sizeof(total), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        cudaFree(rows);
-        return fail(NUFFT3D_ERR_CUDA, std::string("stored H row scan: ") + cudaGetErrorString(e));
-    }
-    const uint64_t entries = (uint64_t)total * 8;
-    const uint64_t bytes = entries * sizeof(int2);
-    if (mode < 0) {
-        size_t fr = 0, to = 0;
-        if (cudaMemGetInfo(&fr, &to) != cudaSuccess || bytes > fr / 2) {
-            cudaGetLastError();
-            cudaFree(rows);
-            return NUFFT3D_SUCCESS;  // evaluate on the fly instead
-        }
-    }
-    int2 *taps = nullptr;
-    const int st = dmalloc(&taps, (size_t)entries, nullptr);
-    if (st != NUFFT3D_SUCCESS) {
-        cudaFree(rows);
-        if (mode < 0) {
-            clear_error();
-            return NUFFT3D_SUCCESS;
-        }
-        return st;
-    }
-    p->tap_rows = rows;
-    p->tap_ent = taps;
-    p->tap_bytes = (int64_t)(bytes + sizeof(uint32_t) * (nnz + 1));
-    p->table_bytes += p->tap_bytes;
-    NUFFT_TRY(launch_tap_fill(p, rows, taps, s));
+    NUFFT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tstore, tb, cnt, rows, (int)(nnz + 1), s));
+    NUFFT_CUDA_TRY(cudaMemcpyAsync(&total, rows + nnz, sizeof(total), cudaMemcpyDeviceToHost, s));
     NUFFT_CUDA_TRY(cudaStreamSynchronize(s));
+    int2 *taps = nullptr;
+    const int st = dmalloc(&taps, (size_t)total * 8, nullptr);
+    if (st != NUFFT3D_SUCCESS) {
+        cudaGetLastError();
+        if (mode > 0) return st;
+        clear_error();
+        return NUFFT3D_SUCCESS;
+    }
+    tmp.push_back(taps);
+    NUFFT_TRY(launch_tap_fill(p, rows, taps, s));
+    *rows_out = rows;
+    *ent = taps;
     return NUFFT3D_SUCCESS;
 }
 
@@ -576,6 +628,16 @@ std::vector<int4> make_pieces(const std::vector<int32_t> &counts, int S)
     // largest pieces first: the heavy centre of radial k-space starts early
     std::stable_sort(blocks.begin(), blocks.end(), [](const int4 &a, const int4 &b) { return a.z > b.z; });
     return blocks;
+}
+
+// Sign of image element i in the stored U: (-1)^(n - N/2) per transformed
+// axis (see grid_index).
+static int deap_sign(const nufft3d_plan *p, size_t i)
+{
+    const size_t N1 = p->N[0], N2 = p->N[1];
+    size_t n = i % N1 + p->N[0] / 2 + i / N1 % N2 + p->N[1] / 2;
+    if (!p->geom.is2d) n += i / (N1 * N2) + p->N[2] / 2;
+    return n & 1 ? -1 : 1;
 }
 
 static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts &o)
@@ -604,13 +666,16 @@ static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts
         kp.T[a] = g.T[a];
         kp.nt[a] = g.nt[a];
         kp.Ra[a] = g.Ra[a];
+        kp.shift[a] = a == 0 ? tile_shift(g) : 0;
     }
     const uint64_t ntiles64 = (uint64_t)g.nt[0] * g.nt[1] * g.nt[2];
-    if (ntiles64 >= 0x7fffffffull) return fail(NUFFT3D_ERR_SIZE, "too many interpolation tiles");
+    kp.slab_cells = slab_cells(g);
+    kp.slabs = slabs_per_tile(g);
+    if (ntiles64 * kp.slabs >= 0x7fffffffull) return fail(NUFFT3D_ERR_SIZE, "too many interpolation tiles");
     kp.ntiles = (uint32_t)ntiles64;
-    const uint32_t ntiles = kp.ntiles;
+    const uint32_t ntiles = kp.ntiles, nslabs = ntiles * (uint32_t)kp.slabs;
 
-    uint32_t *keys = nullptr, *keys_sorted = nullptr;
+    uint64_t *keys = nullptr, *keys_sorted = nullptr;
     int32_t *vals = nullptr;
     NUFFT_TRY(dmalloc(&keys, (size_t)M, nullptr));
     tmp.ptrs.push_back(keys);
@@ -626,7 +691,8 @@ static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts
         NUFFT_CUDA_TRY(cudaGetLastError());
     }
     int end_bit = 1;
-    while ((1ull << end_bit) <= (uint64_t)ntiles) ++end_bit;
+    while ((1ull << end_bit) <= (uint64_t)nslabs) ++end_bit;
+    end_bit += kCurveBits;
     size_t tb = 0;
     NUFFT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys_sorted, vals, p->perm,
                                                    (int)M, 0, end_bit, s));
@@ -636,18 +702,23 @@ static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts
     NUFFT_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tstore, tb, keys, keys_sorted, vals, p->perm,
                                                    (int)M, 0, end_bit, s));
     int32_t *counts = nullptr;
-    NUFFT_TRY(dmalloc(&counts, (size_t)ntiles, nullptr));
+    NUFFT_TRY(dmalloc(&counts, (size_t)nslabs, nullptr));
     tmp.ptrs.push_back(counts);
-    NUFFT_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int32_t) * ntiles, s));
+    NUFFT_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int32_t) * nslabs, s));
     if (M > 0) {
-        k_hist<<<nbM, th, 0, s>>>(keys, M, ntiles, counts);
+        k_hist<<<nbM, th, 0, s>>>(keys, M, nslabs, counts);
         NUFFT_CUDA_TRY(cudaGetLastError());
     }
-    std::vector<int32_t> hc(ntiles);
-    NUFFT_CUDA_TRY(cudaMemcpyAsync(hc.data(), counts, sizeof(int32_t) * ntiles, cudaMemcpyDeviceToHost, s));
+    p->slab_counts.resize(nslabs);
+    NUFFT_CUDA_TRY(
+        cudaMemcpyAsync(p->slab_counts.data(), counts, sizeof(int32_t) * nslabs, cudaMemcpyDeviceToHost, s));
     NUFFT_CUDA_TRY(cudaStreamSynchronize(s));
     int64_t nnz = 0;
-    for (uint32_t t = 0; t < ntiles; ++t) nnz += hc[t];
+    std::vector<int32_t> hc(ntiles, 0);
+    for (uint32_t t = 0; t < nslabs; ++t) {
+        hc[t / kp.slabs] += p->slab_counts[t];
+        nnz += p->slab_counts[t];
+    }
     p->nnz = nnz;
 
     // tile pieces of at most S samples, split evenly
@@ -702,13 +773,20 @@ static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts
         }
     }
     NUFFT_TRY(launch_weight_sum(p, s));
-    NUFFT_TRY(build_tap_table(p, o.tap_table, tmp.ptrs, s));
-    NUFFT_TRY(build_spread_table(p, o.spread_table, s));
+    NUFFT_TRY(build_gather_table(p, o.tap_table, s));
+    if (p->gw && o.spread_table != 0) {
+        uint32_t *rows = nullptr;
+        int2 *ent = nullptr;
+        Tmp taps;  // freed with the build
+        NUFFT_TRY(build_taps(p, o.spread_table, taps.ptrs, &rows, &ent, s));
+        NUFFT_TRY(build_spread_table(p, o.spread_table, rows, ent, s));
+    }
+    std::vector<int32_t>().swap(p->slab_counts);
     // deapodization (FP64 on the host, stored FP32 like deap.m:100-101)
     {
         std::vector<double> U = deap_host(p->N, g.K, p->J, p->alpha, g.radial, g.is2d);
         std::vector<float> Uf(U.size());
-        for (size_t i = 0; i < U.size(); ++i) Uf[i] = (float)U[i];
+        for (size_t i = 0; i < U.size(); ++i) Uf[i] = (float)U[i] * (float)deap_sign(p, i);
         NUFFT_TRY(dmalloc(&p->U, Uf.size(), &p->table_bytes));
         NUFFT_CUDA_TRY(cudaMemcpyAsync(p->U, Uf.data(), sizeof(float) * Uf.size(), cudaMemcpyHostToDevice, s));
         NUFFT_CUDA_TRY(cudaStreamSynchronize(s));
@@ -906,7 +984,7 @@ extern "C" int nufft3d_plan_create(const double *om, int64_t M, const int32_t *N
                     N[0], N[1], N[2], K[0], K[1], K[2], o.J, o.u, alpha, p->radial);
         std::printf("  %lld points (out of %lld) are within bounds; %.2f taps/sample; %lld blocks\n",
                     (long long)p->nnz, (long long)M, p->taps, (long long)p->n_blocks);
-        if (p->tap_ent)
+        if (p->gw)
             std::printf("  stored H: %.1f MB\n", (double)p->tap_bytes / 1e6);
         if (p->spread_ent)
             std::printf("  stored H': %.1f MB\n", (double)p->spread_bytes / 1e6);
@@ -956,8 +1034,12 @@ extern "C" int nufft3d_plan_share(const nufft3d_plan *src, nufft3d_plan **out)
         p->tw[a] = src->tw[a];
         p->fft[a] = src->fft[a];
     }
-    p->tap_rows = src->tap_rows;
-    p->tap_ent = src->tap_ent;
+    p->grecs = src->grecs;
+    p->gchunks = src->gchunks;
+    p->n_gchunks = src->n_gchunks;
+    p->grow = src->grow;
+    p->gw = src->gw;
+    p->gi = src->gi;
     p->tap_bytes = src->tap_bytes;
     p->spread_pieces = src->spread_pieces;
     p->spread_wstart = src->spread_wstart;
@@ -1103,6 +1185,7 @@ extern "C" int nufft3d_get_deap(const nufft3d_plan *p, float *U)
     DeviceGuard guard(p->device);
     const size_t n = (size_t)p->N[0] * p->N[1] * p->N[2];
     NUFFT_CUDA_TRY(cudaMemcpy(U, p->U, n * sizeof(float), cudaMemcpyDeviceToHost));
+    for (size_t i = 0; i < n; ++i) U[i] *= (float)deap_sign(p, i);
     return NUFFT3D_SUCCESS;
 }
 

@@ -110,14 +110,41 @@ constexpr int kSpreadWarps = kBundleWarps;
 constexpr int kSpreadDepth = kBundleDepth;
 constexpr int kMaxBundles = (kTabBuildThreads * kTabSortItems + kRows - 1) / kRows;
 
+// A spread piece takes every stride-th sample of its tile's run (first,
+// first + stride, ...; z of the piece = count | stride << kCountBits): samples
+// of equal position follow one another in the sorted order (the centre of
+// k-space, which every spoke of a radial trajectory samples), and an FP32 sum
+// of many equal terms rounds the same way at every step.  Inside a piece the
+// rows take the samples in a scattered order for the same reason.
+constexpr int kCountBits = 11;
+static_assert(kSpreadCap < (1 << kCountBits), "piece count");
+
+__host__ __device__ __forceinline__ int piece_count(const int4 &pc) { return pc.z & ((1 << kCountBits) - 1); }
+__host__ __device__ __forceinline__ int piece_stride(const int4 &pc) { return pc.z >> kCountBits; }
+
+// A step coprime to n near n/phi: i -> i * step mod n visits 0..n-1 scattered.
+__device__ __forceinline__ int scatter_step(int n)
+{
+    int g = max(1, (int)(0.618034f * (float)n));
+    for (;; ++g) {
+        int a = g, b = n;
+        while (b) {
+            const int t = a % b;
+            a = b;
+            b = t;
+        }
+        if (a == 1) return g;
+    }
+}
+
 // Origin of the padded tile of tile index tid (may be negative or past the
 // grid edge: the grid wraps around).
 __device__ __forceinline__ void tab_tile_origin(const Geom &g, int tid, int &ox, int &oy, int &oz)
 {
-    const int tx = tid % g.nt[0];
-    const int ty = (tid / g.nt[0]) % g.nt[1];
-    const int tz = tid / (g.nt[0] * g.nt[1]);
-    ox = tx * g.T[0] - g.Ra[0];
+    const int tz = tid % g.nt[2];  // z fastest: the tiles of a column are neighbours
+    const int tx = (tid / g.nt[2]) % g.nt[0];
+    const int ty = tid / (g.nt[2] * g.nt[0]);
+    ox = tx * g.T[0] + tile_shift(g) - g.Ra[0];
     oy = ty * g.T[1] - g.Ra[1];
     oz = tz * g.T[2] - g.Ra[2];
 }
@@ -213,7 +240,7 @@ struct TabBuildSmem {
     typename TabSort::TempStorage sort;
     RunLayout<kMaxBundles> L;
     uint16_t srow[kTabBuildThreads * kTabSortItems];  // point of each sorted row
-    int nrows;
+    int nrows, step;
 };
 
 // Plan time, one block per spread piece.  FILL = false: writes the piece's
@@ -240,12 +267,16 @@ k_spread_tab_build(const int4 *__restrict__ pieces, const uint32_t *__restrict__
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < kTabBuildWarps * P; i += blockDim.x) hist[i] = 0;
     __syncthreads();
-    const int s_lo = pc.y + (int)(((long long)pc.z * warp) / kTabBuildWarps);
-    const int s_hi = pc.y + (int)(((long long)pc.z * (warp + 1)) / kTabBuildWarps);
+    const int np = piece_count(pc), stride = piece_stride(pc);
+    const int i_lo = (np * warp) / kTabBuildWarps, i_hi = (np * (warp + 1)) / kTabBuildWarps;
+    if (tid == 0) ss.step = scatter_step(np);
+    __syncthreads();
+    const int step = ss.step;
     uint32_t *h = hist + (size_t)warp * P;
-    for (int s = s_lo; s < s_hi; ++s) {
+    for (int i = i_lo; i < i_hi; ++i) {
+        const int sl = (int)((long long)i * step % np), s = pc.y + sl * stride;
         const size_t r0 = (size_t)__ldg(&rows[s]) * 8, r1 = (size_t)__ldg(&rows[s + 1]) * 8;
-        const uint32_t inc = ((s - pc.y) & 1) ? 0x10000u : 1u;
+        const uint32_t inc = (sl & 1) ? 0x10000u : 1u;
         for (size_t e = r0 + lane; e < r1; e += 32) {
             const int2 t = __ldg(&taps[e]);
             if (t.x != 0) h[t.y] += inc;  // padding entries have weight 0
@@ -345,8 +376,8 @@ k_spread_tab_build(const int4 *__restrict__ pieces, const uint32_t *__restrict__
     }
     // the entries: row slot r starts with parity r & 1, then alternates while
     // both parities last; leftovers follow in sample order
-    for (int s = s_lo; s < s_hi; ++s) {
-        const int sl = s - pc.y, par = sl & 1;
+    for (int i = i_lo; i < i_hi; ++i) {
+        const int sl = (int)((long long)i * step % np), s = pc.y + sl * stride, par = sl & 1;
         const uint32_t inc = par ? 0x10000u : 1u;
         const size_t r0 = (size_t)__ldg(&rows[s]) * 8, r1 = (size_t)__ldg(&rows[s + 1]) * 8;
         for (size_t e = r0 + lane; e < r1; e += 32) {
@@ -369,12 +400,13 @@ k_spread_tab_build(const int4 *__restrict__ pieces, const uint32_t *__restrict__
 // Stage the samples of a piece into one of the two sample buffers (slot
 // 2 + i holds sorted sample first + i) with asynchronous copies; the caller
 // waits for them (cp.async.wait_all) and synchronises before reading.
-__device__ __forceinline__ void stage_samples(const float2 *__restrict__ ks, int nc, int c0, int first, int n,
+__device__ __forceinline__ void stage_samples(const float2 *__restrict__ ks, int nc, int c0, const int4 pc,
                                               unsigned buf_sa)
 {
+    const int first = pc.y, n = piece_count(pc), stride = piece_stride(pc);
     for (int i = threadIdx.x; i < n * 4; i += blockDim.x) {
         const int sl = i >> 2, pr = i & 3;
-        const float2 *src = ks + (size_t)(first + sl) * nc + c0 + 2 * pr;
+        const float2 *src = ks + (size_t)(first + sl * stride) * nc + c0 + 2 * pr;
         const unsigned dst = buf_sa + (unsigned)((sl + 2) * 64 + pr * 16);
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
     }
@@ -421,7 +453,7 @@ k_spread_tab(const float2 *__restrict__ ks, float2 *__restrict__ G, int nc, int 
     uint32_t l_lo = 0, l_hi = 0;
     if (b < npieces) {
         const int4 pc = pieces[b];
-        stage_samples(ks, nc, c0, pc.y, pc.z, ys_sa);
+        stage_samples(ks, nc, c0, pc, ys_sa);
         l_lo = __ldg(&wstart[(size_t)b * (kSpreadWarps + 1) + warp]);
         l_hi = __ldg(&wstart[(size_t)b * (kSpreadWarps + 1) + warp + 1]);
 #pragma unroll
@@ -439,7 +471,7 @@ k_spread_tab(const float2 *__restrict__ ks, float2 *__restrict__ G, int nc, int 
         const int bn = next;
         if (bn < npieces) {
             const int4 pn = pieces[bn];
-            stage_samples(ks, nc, c0, pn.y, pn.z, ys_sa + (unsigned)((buf ^ 1) * kBufF4 * 16));
+            stage_samples(ks, nc, c0, pn, ys_sa + (unsigned)((buf ^ 1) * kBufF4 * 16));
         }
         const char *ys1 = reinterpret_cast<const char *>(ys + buf * kBufF4) + 32 * h + o1;  // first half
         const char *ys2 = ys1 + (o2 - o1);                                                  // second half
@@ -537,16 +569,28 @@ int configure_spread_tab_kernels()
 
 // The stored H' (needs the stored H).  mode 0 = none, 1 = always, -1 = when
 // it takes at most half of the free device memory.
-int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s)
+int build_spread_table(nufft3d_plan *p, int mode, const uint32_t *rows, const int2 *taps, cudaStream_t s)
 {
-    if (mode == 0 || p->tap_ent == nullptr || p->nnz == 0) return NUFFT3D_SUCCESS;
+    if (mode == 0 || taps == nullptr || p->nnz == 0) return NUFFT3D_SUCCESS;
     const Geom &g = p->geom;
     const int P = g.P[0] * g.P[1] * g.P[2];
     if (P > kTabBuildThreads * kTabSortItems || P > 4096 || build_smem(g) > 160 * 1024) {
         if (mode < 0) return NUFFT3D_SUCCESS;
         return fail(NUFFT3D_ERR_UNSUPPORTED, "padded tile too large for the stored H'");
     }
-    std::vector<int4> pcs = make_pieces(p->tile_counts, kSpreadCap);
+    std::vector<int4> pcs;
+    {
+        int64_t off = 0;
+        for (size_t t = 0; t < p->tile_counts.size(); ++t) {
+            const int c = p->tile_counts[t], nb = (c + kSpreadCap - 1) / kSpreadCap;
+            for (int b = 0; b < nb; ++b)
+                pcs.push_back(make_int4((int)t, (int)(off + b), (c - b + nb - 1) / nb | nb << kCountBits, 0));
+            off += c;
+        }
+        // largest pieces first: the heavy centre of radial k-space starts early
+        std::stable_sort(pcs.begin(), pcs.end(),
+                         [](const int4 &a, const int4 &b) { return piece_count(a) > piece_count(b); });
+    }
     const int64_t np = (int64_t)pcs.size();
     pcs.push_back(make_int4(0, 0, 0, 0));
     struct Tmp {
@@ -568,7 +612,7 @@ int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s)
     }
     NUFFT_CUDA_TRY(cudaMemcpyAsync(dp, pcs.data(), sizeof(int4) * pcs.size(), cudaMemcpyHostToDevice, s));
     const size_t smem = build_smem(g);
-    k_spread_tab_build<false><<<(unsigned)np, kTabBuildThreads, smem, s>>>(dp, p->tap_rows, p->tap_ent, g, dl,
+    k_spread_tab_build<false><<<(unsigned)np, kTabBuildThreads, smem, s>>>(dp, rows, taps, g, dl,
                                                                          nullptr, nullptr);
     NUFFT_CUDA_TRY(cudaGetLastError());
     std::vector<uint32_t> nl((size_t)np);
@@ -617,7 +661,7 @@ int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s)
     p->spread_bytes = (int64_t)(bytes + wbytes + sizeof(int4) * pcs.size());
     p->table_bytes += p->spread_bytes;
     NUFFT_CUDA_TRY(cudaMemcpyAsync(pieces, pcs.data(), sizeof(int4) * pcs.size(), cudaMemcpyHostToDevice, s));
-    k_spread_tab_build<true><<<(unsigned)np, kTabBuildThreads, smem, s>>>(pieces, p->tap_rows, p->tap_ent, g,
+    k_spread_tab_build<true><<<(unsigned)np, kTabBuildThreads, smem, s>>>(pieces, rows, taps, g,
                                                                         nullptr, wst, ent);
     NUFFT_CUDA_TRY(cudaGetLastError());
     NUFFT_CUDA_TRY(cudaStreamSynchronize(s));
