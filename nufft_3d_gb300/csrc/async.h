@@ -120,6 +120,12 @@ __device__ __forceinline__ void prefetch_line(const void *p)
     asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
 }
 
+// The same for bytes (a multiple of 16) from p on, by the bulk copy unit.
+__device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // Streaming loads of table entries (read once: no L1 allocation).
 __device__ __forceinline__ float4 ld_stream4(const float4 *p)
 {
@@ -127,6 +133,13 @@ __device__ __forceinline__ float4 ld_stream4(const float4 *p)
     asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                  : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ unsigned ld_stream16(const uint16_t *p)
+{
+    uint16_t v;
+    asm volatile("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(v) : "l"(p));
     return v;
 }
 

@@ -43,7 +43,7 @@ using namespace nufft3d;
 struct nufft3d_batch {
     int device = 0, nvol = 0, R = 0, radial = 1, is2d = 0, cb = 8;
     bool rare = false;
-    bool stored_h = false;  // every volume's plan holds its stored H
+    bool stored_h = false, stored_ht = false;  // every volume's plan holds its stored H, its stored H'
     std::vector<nufft3d_plan *> plans;
     std::vector<int> nc;
     // descriptor arrays (device) and their host mirrors
@@ -428,6 +428,13 @@ static int run_interp(nufft3d_batch *b, bool gather, cudaStream_t s)
         }
         return NUFFT3D_SUCCESS;
     }
+    if (!gather && b->stored_ht) {
+        for (int v = 0; v < b->nvol; ++v) {
+            const BatchInterp &g = b->h_spr[v];
+            NUFFT_TRY(launch_spread(b->plans[v], g.in, g.out, g.nc, s));
+        }
+        return NUFFT3D_SUCCESS;
+    }
     for (auto &g : b->igroups)
         NUFFT_TRY(launch_interp_batch(gather, g.cb, b->R, b->radial, gather ? b->gat : b->spr, g.tab, g.n, g.smem,
                                       b->plans[0]->kb, b->work, b->plans[0]->sm_count, s));
@@ -587,8 +594,9 @@ extern "C" int nufft3d_batch_create(nufft3d_plan *const *plans, const int *nc, i
             d.kb = p->kb;
             d.cand = p->cand_desc;
             d.status = plan_status(p);  // timeouts are reported on the volume's plan
-            if (v == 0) b->stored_h = true;
-            if (!p->gw) b->stored_h = false;
+            if (v == 0) b->stored_h = b->stored_ht = true;
+            if (p->nnz > 0 && !p->gw) b->stored_h = false;
+            if (p->nnz > 0 && !p->spread_ent) b->stored_ht = false;
             d.nc = nc[v];
             b->h_gat[v] = d;
             b->h_spr[v] = d;

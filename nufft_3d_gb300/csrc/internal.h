@@ -198,9 +198,9 @@ inline int slabs_per_tile(const Geom &g) { return g.is2d ? 1 : g.T[2] / 2; }
 // Slots of a plan's small device work buffer (int[16]).
 constexpr int kWorkGather = 0;   // work counter of the persistent gather
 constexpr int kWorkSpread = 1;   // work counter of the persistent spread
-constexpr int kWorkTapFill = 2;  // stored-H build: fill disagrees with count
 constexpr int kWorkStatus = 3;   // interpolation status (a bounded wait expired)
 constexpr int kWorkGatherTab = 4;  // [2] stored-H gather: next chunk, blocks done (the last one clears both)
+constexpr int kWorkSpreadTab = 6;  // [2] the same of the stored-H' spread
 constexpr int kDefaultWaitPolls = 1 << 22;
 
 struct BatchInterp {
@@ -350,12 +350,15 @@ struct nufft3d_plan {
     float4 *gw = nullptr;
     uint32_t *gi = nullptr;
     int64_t tap_bytes = 0;
-    // stored H' for the 8-coil spread (tables.cu): pieces of at most
-    // kSpreadCap samples, (tile, first sample, count, first line); the warps'
-    // first lines (33 per piece); the bundles of 128-byte lines
+    // stored H' (tables.cu): pieces (first sample, count and stride, first
+    // step, first slab), the warps' first steps and segments, the lines'
+    // weights and slots, the segments' grid points and steps
     int4 *spread_pieces = nullptr;
-    uint32_t *spread_wstart = nullptr;
-    int2 *spread_ent = nullptr;
+    uint2 *spread_wstart = nullptr;
+    float4 *spread_ent = nullptr;
+    uint16_t *spread_idx = nullptr, *spread_steps = nullptr;
+    int4 *spread_pts = nullptr;
+    int spread_cap = 0;          // most samples of a piece
     int64_t n_spread_pieces = 0;
     int64_t spread_bytes = 0;
     int threads = 256;
@@ -402,10 +405,6 @@ int launch_gather(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, float sc
                   const float *wsample, cudaStream_t s);
 // plan time: per-block bound on summed weights (blocks[b].w) for the spread
 int launch_weight_sum(nufft3d_plan *p, cudaStream_t s);
-// plan time, entries for the build of the stored H': rows[s] = chunks of 8
-// entries in sample s's row, then the entries (rows = chunk offsets)
-int launch_tap_count(nufft3d_plan *p, uint32_t *rows, cudaStream_t s);
-int launch_tap_fill(nufft3d_plan *p, const uint32_t *rows, int2 *taps, cudaStream_t s);
 // the stored tables serve this plan (8-coil passes, R <= 3)
 bool tap_table_applies(const nufft3d_plan *p);
 // stored H (gather_tab.cu): plan-time build, and the gather of coils
@@ -421,11 +420,10 @@ int launch_spread(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, cudaStre
 // Largest spread piece of the stored H' (samples staged in shared memory,
 // two pieces at a time).
 constexpr int kSpreadCap = 1664;
-// stored H' (tables.cu): plan-time build from the stored H, the 8-coil
-// spread pass that reads it, and whether it serves coils c0..c0+7 of nc
-int build_spread_table(nufft3d_plan *p, int mode, const uint32_t *rows, const int2 *taps, cudaStream_t s);
-int launch_spread_tab(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, int c0, cudaStream_t s);
-bool spread_tab_applies(const nufft3d_plan *p, int nc, int c0);
+// stored H' (tables.cu): plan-time build, and the spread of coils
+// c0..c0+cb-1 that reads it (cb 1, 2, 4 or 8)
+int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s);
+int launch_spread_tab(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, int c0, int cb, cudaStream_t s);
 int configure_spread_tab_kernels();
 // multiprocessors the persistent interpolation kernels of a handle may use
 int interp_grid_sms(const nufft3d_plan *p);

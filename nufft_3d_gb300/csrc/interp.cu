@@ -901,143 +901,6 @@ k_weight_sum(const float4 *__restrict__ samples, int4 *__restrict__ blocks, Geom
     if (threadIdx.x == 0) blocks[blockIdx.x].w = __float_as_int(m * 1.001f + 1e-3f);
 }
 
-// ------------------------------------------- entries for the stored H' build
-// Weight and tile offset of candidate ci for the stored H.  The distance is
-// formed with explicitly rounded operations (never contracted into FMAs), so
-// the count and fill passes, compiled separately, take identical support
-// decisions.
-template <bool RADIAL>
-__device__ __forceinline__ bool tap_exact(int ci, const SampleGeo &g, const CandSmem &cs, const KBParams &kb,
-                                          float &w, int &off)
-{
-    const float4 cf = cs.f[g.lbase + ci];
-    const float ex = __fsub_rn(cf.x, g.fx), ey = __fsub_rn(cf.y, g.fy), ez = __fsub_rn(cf.z, g.fz);
-    const float ex2 = __fmul_rn(ex, ex), ey2 = __fmul_rn(ey, ey), ez2 = __fmul_rn(ez, ez);
-    const float h2 = kb.half2;
-    if (RADIAL) {
-        const float d2 = __fadd_rn(__fadd_rn(ez2, ey2), ex2);
-        if (!(d2 <= h2)) return false;
-        w = kb_weight(d2, kb);
-    } else {
-        if (!(ex2 <= h2 && ey2 <= h2 && ez2 <= h2)) return false;
-        w = __fmul_rn(__fmul_rn(kb_weight(ez2, kb), kb_weight(ey2, kb)), kb_weight(ex2, kb));
-    }
-    off = tap_offset(cf, g);
-    return true;
-}
-
-// Plan time, pass 1 of the stored H: rows[s] = 8-entry chunks of sample s's
-// row (its hits, rounded up).  One warp per sample.
-template <bool RADIAL>
-__global__ void __launch_bounds__(256)
-k_tap_count(const float4 *__restrict__ samples, int64_t nnz, Geom g, KBParams kb, const __grid_constant__ Cand cd,
-            uint32_t *__restrict__ rows)
-{
-    extern __shared__ float4 smem4[];
-    CandSmem cs;
-    carve_cand(cd, cs, smem4);
-    build_cand(cd, cs);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nnz; s += nw) {
-        const SampleGeo sg = sample_geo(__ldg(&samples[s]), g.P[0], g.P[1], cs);
-        int nh = 0;
-        for (int base = 0; base < sg.ln; base += 32) {
-            const int ci = base + lane;
-            float w;
-            int off;
-            const bool hit = ci < sg.ln && tap_exact<RADIAL>(ci, sg, cs, kb, w, off);
-            nh += __popc(__ballot_sync(0xffffffffu, hit));
-        }
-        if (lane == 0) rows[s] = (uint32_t)((nh + 7) >> 3);
-    }
-}
-
-// Plan time, pass 2: the entries of every row in bank order (see above).
-// Per warp two shared buffers of cap entries: the hits in candidate order,
-// then in round-robin residue order.  *err is set if a row has more hits
-// than the count pass found (the row is then cut at its length).
-template <bool RADIAL>
-__global__ void __launch_bounds__(256)
-k_tap_fill(const float4 *__restrict__ samples, int64_t nnz, Geom g, KBParams kb, const __grid_constant__ Cand cd,
-           const uint32_t *__restrict__ rows, int2 *__restrict__ taps, int cap, int *__restrict__ err)
-{
-    extern __shared__ float4 smem4[];
-    CandSmem cs;
-    int2 *bufs = reinterpret_cast<int2 *>(carve_cand(cd, cs, smem4));
-    build_cand(cd, cs);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int2 *A = bufs + (size_t)warp * 2 * cap, *B = A + cap;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nnz; s += nw) {
-        const SampleGeo sg = sample_geo(__ldg(&samples[s]), g.P[0], g.P[1], cs);
-        int nh = 0;
-        for (int base = 0; base < sg.ln; base += 32) {
-            const int ci = base + lane;
-            float w = 0.f;
-            int off = 0;
-            const bool hit = ci < sg.ln && tap_exact<RADIAL>(ci, sg, cs, kb, w, off);
-            const unsigned m = __ballot_sync(0xffffffffu, hit);
-            if (hit) A[nh + __popc(m & ((1u << lane) - 1u))] = make_int2(__float_as_int(w), off);
-            nh += __popc(m);
-        }
-        __syncwarp();
-        // the row holds what the count pass found; never write past it
-        const size_t row = (size_t)__ldg(&rows[s]) * 8;
-        const int nfill = (int)((size_t)__ldg(&rows[s + 1]) * 8 - row);
-        if (nh > nfill) {
-            if (lane == 0) atomicOr(err, 1);
-            nh = nfill;
-        }
-        // hits per residue of the tile offset mod 8
-        int cnt = 0;
-        if (lane < 8)
-            for (int i = 0; i < nh; ++i) cnt += (A[i].y & 7) == lane;
-        int n[8];
-#pragma unroll
-        for (int r = 0; r < 8; ++r) n[r] = __shfl_sync(0xffffffffu, cnt, r);
-        // round-robin order: level k holds the k-th hit of every residue that
-        // has one, the residues with more hits first (they run out last)
-        for (int i = lane; i < nh; i += 32) {
-            const int2 e = A[i];
-            const int r = e.y & 7;
-            int rank = 0;
-            for (int i2 = 0; i2 < i; ++i2) rank += (A[i2].y & 7) == r;
-            int nr = 0;
-#pragma unroll
-            for (int r2 = 0; r2 < 8; ++r2) nr = r2 == r ? n[r2] : nr;
-            int pos = 0;
-#pragma unroll
-            for (int r2 = 0; r2 < 8; ++r2) {
-                const bool before = n[r2] > nr || (n[r2] == nr && r2 < r);
-                pos += min(n[r2], rank) + ((before && n[r2] > rank) ? 1 : 0);
-            }
-            B[pos] = e;
-        }
-        __syncwarp();
-        // inside each chunk: even offsets first, then odd ones; zero padding
-        for (int p = lane; p < nfill; p += 32) {
-            if (p >= nh) {
-                taps[row + p] = make_int2(0, 0);
-                continue;
-            }
-            const int c8 = p & ~7, end = min(c8 + 8, nh);
-            int ev = 0, evb = 0;
-            for (int k = c8; k < end; ++k) {
-                const int even = (B[k].y & 1) == 0;
-                ev += even;
-                evb += (k < p) ? even : 0;
-            }
-            const int2 e = B[p];
-            const int slot = (e.y & 1) ? ev + ((p - c8) - evb) : evb;
-            taps[row + c8 + slot] = e;
-        }
-        __syncwarp();  // A and B are refilled for the next sample
-    }
-}
-
 // user layout [M][nc] (coil-major) <-> sorted [nnz][nc] (coil fastest); the
 // sorted side is read/written as one contiguous nc-vector per sample.
 __global__ void k_permute_out(const float2 *__restrict__ ks, float2 *__restrict__ k,
@@ -1343,6 +1206,8 @@ static int dispatch(nufft3d_plan *p, const float2 *in, float2 *out, int nc, int 
                           : dispatch_r<GATHER, CB, false>(p, in, out, nc, c0, scale, ws, s);
 }
 
+constexpr int64_t kSpreadTabSamples = 32768;
+
 template <bool GATHER>
 static int interp(nufft3d_plan *p, const float2 *in, float2 *out, int nc, float scale,
                   const float *ws, cudaStream_t s)
@@ -1359,17 +1224,20 @@ static int interp(nufft3d_plan *p, const float2 *in, float2 *out, int nc, float 
             if (cb > rem) break;
             continue;
         }
+        // The stored H', where its FP32 sums, whose last bits depend on the order
+        // in which pieces meet in the grid, buy time: plans of fewer samples and
+        // coils keep the fixed-point spread, whose sums at those sizes are exact
+        // and equal bit for bit from call to call.
+        if (!GATHER && p->spread_ent && (cb >= 8 || p->nnz >= kSpreadTabSamples)) {
+            NUFFT_TRY(launch_spread_tab(p, in, out, nc, c0, cb, s));
+            if (cb > rem) break;
+            continue;
+        }
         switch (cb) {
         case 1: st = dispatch<GATHER, 1>(p, in, out, nc, c0, scale, ws, s); break;
         case 2: st = dispatch<GATHER, 2>(p, in, out, nc, c0, scale, ws, s); break;
         case 4: st = dispatch<GATHER, 4>(p, in, out, nc, c0, scale, ws, s); break;
-        default:
-            // the stored H' serves the spread of full passes of an even coil count
-            if (!GATHER && spread_tab_applies(p, nc, c0))
-                st = launch_spread_tab(p, in, out, nc, c0, s);
-            else
-                st = dispatch<GATHER, 8>(p, in, out, nc, c0, scale, ws, s);
-            break;
+        default: st = dispatch<GATHER, 8>(p, in, out, nc, c0, scale, ws, s); break;
         }
         if (st != NUFFT3D_SUCCESS) return st;
         if (cb > rem) break;
@@ -1388,41 +1256,6 @@ int launch_weight_sum(nufft3d_plan *p, cudaStream_t s)
         k_weight_sum<false><<<(unsigned)p->n_blocks, kInterpThreads, smem, s>>>(p->samples, p->blocks, p->geom,
                                                                              p->kb, cand_of(p));
     NUFFT_CUDA_TRY(cudaGetLastError());
-    return NUFFT3D_SUCCESS;
-}
-
-int launch_tap_count(nufft3d_plan *p, uint32_t *rows, cudaStream_t s)
-{
-    if (p->nnz == 0) return NUFFT3D_SUCCESS;
-    const size_t smem = cand_smem_bytes(p->n_cand);
-    const unsigned nb = (unsigned)std::min<int64_t>((p->nnz + 7) / 8, (int64_t)p->sm_count * 8);
-    if (p->geom.radial)
-        k_tap_count<true><<<nb, 256, smem, s>>>(p->samples, p->nnz, p->geom, p->kb, cand_of(p), rows);
-    else
-        k_tap_count<false><<<nb, 256, smem, s>>>(p->samples, p->nnz, p->geom, p->kb, cand_of(p), rows);
-    NUFFT_CUDA_TRY(cudaGetLastError());
-    return NUFFT3D_SUCCESS;
-}
-
-int launch_tap_fill(nufft3d_plan *p, const uint32_t *rows, int2 *taps, cudaStream_t s)
-{
-    if (p->nnz == 0) return NUFFT3D_SUCCESS;
-    int *err = p->work + kWorkTapFill;  // the plan's own flag (plans may be built concurrently)
-    NUFFT_CUDA_TRY(cudaMemsetAsync(err, 0, sizeof(int), s));
-    int cap = 0;
-    for (int q = 0; q < 8; ++q) cap = std::max(cap, p->cand_desc.cnt[q]);
-    const size_t smem = cand_smem_bytes(p->n_cand) + (size_t)8 * 2 * cap * sizeof(int2);
-    if (smem > 200 * 1024) return fail(NUFFT3D_ERR_UNSUPPORTED, "candidate lists too long for the stored H");
-    const unsigned nb = (unsigned)std::min<int64_t>((p->nnz + 7) / 8, (int64_t)p->sm_count * 8);
-    if (p->geom.radial)
-        k_tap_fill<true><<<nb, 256, smem, s>>>(p->samples, p->nnz, p->geom, p->kb, cand_of(p), rows, taps, cap, err);
-    else
-        k_tap_fill<false><<<nb, 256, smem, s>>>(p->samples, p->nnz, p->geom, p->kb, cand_of(p), rows, taps, cap, err);
-    NUFFT_CUDA_TRY(cudaGetLastError());
-    int herr = 0;
-    NUFFT_CUDA_TRY(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    NUFFT_CUDA_TRY(cudaStreamSynchronize(s));
-    if (herr) return fail(NUFFT3D_ERR_CUDA, "stored H: fill pass disagrees with the count pass");
     return NUFFT3D_SUCCESS;
 }
 
@@ -1551,10 +1384,6 @@ int configure_interp_kernels()
 {
     NUFFT_TRY(allow_smem(k_weight_sum<true>));
     NUFFT_TRY(allow_smem(k_weight_sum<false>));
-    NUFFT_TRY(allow_smem(k_tap_count<true>));
-    NUFFT_TRY(allow_smem(k_tap_count<false>));
-    NUFFT_TRY(allow_smem(k_tap_fill<true>));
-    NUFFT_TRY(allow_smem(k_tap_fill<false>));
     NUFFT_TRY(cfg_cb<1>());
     NUFFT_TRY(cfg_cb<2>());
     NUFFT_TRY(cfg_cb<4>());

@@ -22,7 +22,6 @@
 #include <vector>
 
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
 
 #include "bank_order.h"
 #include "internal.h"
@@ -490,7 +489,8 @@ static void adopt_tables(nufft3d_plan *p)
     auto t = std::make_shared<TableOwner>();
     t->device = p->device;
     t->ptrs = {p->samples, p->perm, p->inv, p->blocks, p->cand, p->U, p->d, p->d_orig,
-               p->tw[0], p->tw[1], p->tw[2], p->grecs, p->gchunks, p->grow, p->gw, p->gi, p->spread_pieces, p->spread_wstart, p->spread_ent};
+               p->tw[0], p->tw[1], p->tw[2], p->grecs, p->gchunks, p->grow, p->gw, p->gi, p->spread_pieces, p->spread_wstart, p->spread_ent, p->spread_idx,
+               p->spread_pts, p->spread_steps};
     p->tables = t;
 }
 
@@ -519,6 +519,9 @@ static void free_plan_memory(nufft3d_plan *p)
         F(p->spread_pieces);
         F(p->spread_wstart);
         F(p->spread_ent);
+        F(p->spread_idx);
+        F(p->spread_pts);
+        F(p->spread_steps);
     }
     F(p->wbuf);
     F(p->work);
@@ -561,52 +564,6 @@ static int dmalloc(T **ptr, size_t count, int64_t *acc)
         return fail(NUFFT3D_ERR_NOMEM, std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
     }
     if (acc) *acc += (int64_t)(count * sizeof(T));
-    return NUFFT3D_SUCCESS;
-}
-
-// The taps of every sample in tile order, (weight bits, tile offset) in rows
-// padded to whole chunks of 8, from which the stored H' is built: count each
-// row's chunks, scan them into row offsets, then fill the rows.  *ent stays
-// null where the memory does not suffice and mode allows to do without.
-static int build_taps(nufft3d_plan *p, int mode, std::vector<void *> &tmp, uint32_t **rows_out, int2 **ent,
-                      cudaStream_t s)
-{
-    const int64_t nnz = p->nnz;
-    int maxcnt = 0;
-    for (int q = 0; q < 8; ++q) maxcnt = std::max(maxcnt, p->cand_desc.cnt[q]);
-    if ((uint64_t)nnz * (uint64_t)((maxcnt + 7) / 8) >= 0xffffffffull) {  // row offsets are 32-bit chunk indices
-        if (mode < 0) return NUFFT3D_SUCCESS;
-        return fail(NUFFT3D_ERR_SIZE, "too many samples for the stored H'");
-    }
-    uint32_t *cnt = nullptr;
-    NUFFT_TRY(dmalloc(&cnt, (size_t)nnz + 1, nullptr));
-    tmp.push_back(cnt);
-    NUFFT_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * (nnz + 1), s));
-    NUFFT_TRY(launch_tap_count(p, cnt, s));
-    size_t tb = 0;
-    NUFFT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, cnt, (int)(nnz + 1), s));
-    void *tstore = nullptr;
-    NUFFT_TRY(dmalloc((char **)&tstore, tb ? tb : 1, nullptr));
-    tmp.push_back(tstore);
-    uint32_t *rows = nullptr;
-    NUFFT_TRY(dmalloc(&rows, (size_t)nnz + 1, nullptr));
-    tmp.push_back(rows);
-    uint32_t total = 0;
-    NUFFT_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tstore, tb, cnt, rows, (int)(nnz + 1), s));
-    NUFFT_CUDA_TRY(cudaMemcpyAsync(&total, rows + nnz, sizeof(total), cudaMemcpyDeviceToHost, s));
-    NUFFT_CUDA_TRY(cudaStreamSynchronize(s));
-    int2 *taps = nullptr;
-    const int st = dmalloc(&taps, (size_t)total * 8, nullptr);
-    if (st != NUFFT3D_SUCCESS) {
-        cudaGetLastError();
-        if (mode > 0) return st;
-        clear_error();
-        return NUFFT3D_SUCCESS;
-    }
-    tmp.push_back(taps);
-    NUFFT_TRY(launch_tap_fill(p, rows, taps, s));
-    *rows_out = rows;
-    *ent = taps;
     return NUFFT3D_SUCCESS;
 }
 
@@ -774,13 +731,7 @@ static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts
     }
     NUFFT_TRY(launch_weight_sum(p, s));
     NUFFT_TRY(build_gather_table(p, o.tap_table, s));
-    if (p->gw && o.spread_table != 0) {
-        uint32_t *rows = nullptr;
-        int2 *ent = nullptr;
-        Tmp taps;  // freed with the build
-        NUFFT_TRY(build_taps(p, o.spread_table, taps.ptrs, &rows, &ent, s));
-        NUFFT_TRY(build_spread_table(p, o.spread_table, rows, ent, s));
-    }
+    NUFFT_TRY(build_spread_table(p, o.spread_table, s));
     std::vector<int32_t>().swap(p->slab_counts);
     // deapodization (FP64 on the host, stored FP32 like deap.m:100-101)
     {
@@ -1044,6 +995,10 @@ extern "C" int nufft3d_plan_share(const nufft3d_plan *src, nufft3d_plan **out)
     p->spread_pieces = src->spread_pieces;
     p->spread_wstart = src->spread_wstart;
     p->spread_ent = src->spread_ent;
+    p->spread_idx = src->spread_idx;
+    p->spread_pts = src->spread_pts;
+    p->spread_steps = src->spread_steps;
+    p->spread_cap = src->spread_cap;
     p->n_spread_pieces = src->n_spread_pieces;
     p->spread_bytes = src->spread_bytes;
     p->table_bytes = src->table_bytes;
