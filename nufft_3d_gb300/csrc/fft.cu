@@ -15,8 +15,10 @@
 // Forward: FX (image*U -> B1), FY (B1 -> B2), FZ (B2 -> G).
 // Adjoint: IZ (G -> B2), IY (B2 -> B1), IX (B1 -> image, *U*scale).
 //
-// Each block runs a mixed-radix Stockham FFT (radix 2,3,4,5,7,8,11,13) on a
-// batch of lines held in shared memory; the inverse is conj(FFT(conj(x))).
+// A length that is a product of two register DFTs (2 to 32 points) runs as two
+// phases in registers with one exchange through shared memory; other lengths
+// run a mixed-radix Stockham FFT (radix 2,3,4,5,7,8,11,13) on lines held in
+// shared memory.  The inverse is conj(FFT(conj(x))).
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -35,25 +37,47 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(
 // multiply by -i
 __device__ __forceinline__ float2 cmi(float2 a) { return make_float2(a.y, -a.x); }
 
-template <int R>
-__device__ __forceinline__ void dft(float2 (&u)[R], const float2 *__restrict__ tw, int n)
+// exp(-2 pi i j / n), n = 2..kMaxRadix, filled once per device from FP64 values;
+// indexed at compile time, so the twiddles are operands from constant memory.
+constexpr int kMaxRadix = 32;
+__constant__ float2 c_w[kMaxRadix * (kMaxRadix + 1) / 2];
+
+template <int N>
+__device__ __forceinline__ float2 wconst(int j)
 {
-    // generic small prime: y_q = sum_t u_t W_R^{qt}, W from the length-n table
-    float2 y[R];
-    const int step = n / R;
+    return c_w[N * (N - 1) / 2 + j];
+}
+
+// Odd prime: inputs t and R - t share their cosines and (negated) sines, so an
+// output pair (q, R - q) takes R - 1 real products a component.
+template <int R>
+__device__ __forceinline__ void dft(float2 (&u)[R])
+{
+    constexpr int H = R / 2;
+    float2 a[H], b[H], y0 = u[0];
 #pragma unroll
-    for (int q = 0; q < R; ++q) {
-        float2 acc = u[0];
-#pragma unroll
-        for (int t = 1; t < R; ++t) acc = cadd(acc, cmul(u[t], __ldg(&tw[((q * t) % R) * step])));
-        y[q] = acc;
+    for (int t = 1; t <= H; ++t) {
+        a[t - 1] = cadd(u[t], u[R - t]);
+        b[t - 1] = csub(u[t], u[R - t]);
+        y0 = cadd(y0, a[t - 1]);
     }
 #pragma unroll
-    for (int q = 0; q < R; ++q) u[q] = y[q];
+    for (int q = 1; q <= H; ++q) {
+        float2 m = u[0], s = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int t = 1; t <= H; ++t) {
+            const float2 w = wconst<R>((q * t) % R);
+            m = make_float2(fmaf(w.x, a[t - 1].x, m.x), fmaf(w.x, a[t - 1].y, m.y));
+            s = make_float2(fmaf(w.y, b[t - 1].x, s.x), fmaf(w.y, b[t - 1].y, s.y));
+        }
+        u[q] = make_float2(m.x - s.y, m.y + s.x);
+        u[R - q] = make_float2(m.x + s.y, m.y - s.x);
+    }
+    u[0] = y0;
 }
 
 template <>
-__device__ __forceinline__ void dft<2>(float2 (&u)[2], const float2 *__restrict__, int)
+__device__ __forceinline__ void dft<2>(float2 (&u)[2])
 {
     float2 a = u[0], b = u[1];
     u[0] = cadd(a, b);
@@ -61,7 +85,7 @@ __device__ __forceinline__ void dft<2>(float2 (&u)[2], const float2 *__restrict_
 }
 
 template <>
-__device__ __forceinline__ void dft<3>(float2 (&u)[3], const float2 *__restrict__, int)
+__device__ __forceinline__ void dft<3>(float2 (&u)[3])
 {
     const float s3 = 0.86602540378443864676f; // sin(2 pi / 3)
     float2 t = cadd(u[1], u[2]);
@@ -75,7 +99,7 @@ __device__ __forceinline__ void dft<3>(float2 (&u)[3], const float2 *__restrict_
 }
 
 template <>
-__device__ __forceinline__ void dft<4>(float2 (&u)[4], const float2 *__restrict__, int)
+__device__ __forceinline__ void dft<4>(float2 (&u)[4])
 {
     float2 t0 = cadd(u[0], u[2]), t1 = csub(u[0], u[2]);
     float2 t2 = cadd(u[1], u[3]), t3 = cmi(csub(u[1], u[3]));
@@ -86,7 +110,7 @@ __device__ __forceinline__ void dft<4>(float2 (&u)[4], const float2 *__restrict_
 }
 
 template <>
-__device__ __forceinline__ void dft<5>(float2 (&u)[5], const float2 *__restrict__, int)
+__device__ __forceinline__ void dft<5>(float2 (&u)[5])
 {
     const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
     const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
@@ -106,13 +130,13 @@ __device__ __forceinline__ void dft<5>(float2 (&u)[5], const float2 *__restrict_
 }
 
 template <>
-__device__ __forceinline__ void dft<8>(float2 (&u)[8], const float2 *__restrict__ tw, int n)
+__device__ __forceinline__ void dft<8>(float2 (&u)[8])
 {
     // radix-2 split: evens and odds through radix-4, combined with W8^k
     float2 e[4] = {u[0], u[2], u[4], u[6]};
     float2 o[4] = {u[1], u[3], u[5], u[7]};
-    dft<4>(e, tw, n);
-    dft<4>(o, tw, n);
+    dft<4>(e);
+    dft<4>(o);
     const float h = 0.70710678118654752440f;
     float2 o1 = make_float2(h * (o[1].x + o[1].y), h * (o[1].y - o[1].x)); // * (1-i)/sqrt2
     float2 o2 = cmi(o[2]);                                                   // * -i
@@ -150,7 +174,7 @@ __device__ __forceinline__ void fft_stage(const float2 *__restrict__ a, float2 *
 #pragma unroll
             for (int q = 1; q < R; ++q) u[q] = cmul(u[q], __ldg(&tw[q * k * twstep]));
         }
-        dft<R>(u, tw, n);
+        dft<R>(u);
         const int j = (i - k) * R + k;
 #pragma unroll
         for (int q = 0; q < R; ++q) dst[j + q * p] = u[q];
@@ -203,21 +227,10 @@ __device__ __forceinline__ int slot_of(int n, int N, int K)
 }
 
 // ------------------------------------------------ four-step line passes
-// In-register DFTs of 12, 16, 20 and 24 points built from the radix 3/4/5/8
-// butterflies (n = B*a + b, k = ka + A*kb), with the W_AB twiddles read from
-// constant memory at compile-time indices (tables filled once per device from
-// FP64 values).
-__constant__ float2 c_w12[12];
-__constant__ float2 c_w16[16];
-__constant__ float2 c_w20[20];
-__constant__ float2 c_w24[24];
-
-template <int N>
-__device__ __forceinline__ float2 wconst(int j);
-template <> __device__ __forceinline__ float2 wconst<12>(int j) { return c_w12[j]; }
-template <> __device__ __forceinline__ float2 wconst<16>(int j) { return c_w16[j]; }
-template <> __device__ __forceinline__ float2 wconst<20>(int j) { return c_w20[j]; }
-template <> __device__ __forceinline__ float2 wconst<24>(int j) { return c_w24[j]; }
+// In-register DFTs of composite lengths (n = B*a + b, k = ka + A*kb), the
+// W_AB twiddles from constant memory.
+template <int R>
+__device__ __forceinline__ void dft_reg(float2 (&u)[R]);
 
 template <int A, int B>
 __device__ __forceinline__ void dft_comp(float2 (&u)[A * B])
@@ -228,7 +241,7 @@ __device__ __forceinline__ void dft_comp(float2 (&u)[A * B])
         float2 v[A];
 #pragma unroll
         for (int a = 0; a < A; ++a) v[a] = u[B * a + b];
-        dft<A>(v, nullptr, 0);
+        dft_reg<A>(v);
 #pragma unroll
         for (int ka = 0; ka < A; ++ka) {
             float2 x = v[ka];
@@ -241,19 +254,28 @@ __device__ __forceinline__ void dft_comp(float2 (&u)[A * B])
         float2 v[B];
 #pragma unroll
         for (int b = 0; b < B; ++b) v[b] = t[b * A + ka];
-        dft<B>(v, nullptr, 0);
+        dft_reg<B>(v);
 #pragma unroll
         for (int kb = 0; kb < B; ++kb) u[ka + A * kb] = v[kb];
     }
 }
 
+// first factor of a register DFT, 1 for the butterflies
+__host__ __device__ constexpr int dft_split(int r)
+{
+    return r == 6 || r == 10 || r == 14 || r == 22 || r == 26 ? 2
+         : r == 9 || r == 12 || r == 15 || r == 18 || r == 21 || r == 24 || r == 27 ? 3
+         : r == 16 || r == 20 || r == 28 || r == 32 ? 4
+         : r == 25 || r == 30 ? 5 : 1;
+}
+
 template <int R>
-__device__ __forceinline__ void dft_reg(float2 (&u)[R]);
-template <> __device__ __forceinline__ void dft_reg<8>(float2 (&u)[8]) { dft<8>(u, nullptr, 0); }
-template <> __device__ __forceinline__ void dft_reg<12>(float2 (&u)[12]) { dft_comp<3, 4>(u); }
-template <> __device__ __forceinline__ void dft_reg<16>(float2 (&u)[16]) { dft_comp<4, 4>(u); }
-template <> __device__ __forceinline__ void dft_reg<20>(float2 (&u)[20]) { dft_comp<4, 5>(u); }
-template <> __device__ __forceinline__ void dft_reg<24>(float2 (&u)[24]) { dft_comp<3, 8>(u); }
+__device__ __forceinline__ void dft_reg(float2 (&u)[R])
+{
+    constexpr int A = dft_split(R);
+    if constexpr (A == 1) dft<R>(u);
+    else dft_comp<A, R / A>(u);
+}
 
 // Strided pass (y or z) for K = R1 * 16 over lp.vec = 16 contiguous lines:
 // X[k1 + R1 k2] = sum_n2 W16^(n2 k2) W_K^(n2 k1) sum_n1 x[16 n1 + n2] W_R1^(n1 k1).
@@ -496,20 +518,270 @@ static int launch_line4(int r1, const float2 *in, float2 *out, const LinePass &l
     return NUFFT3D_SUCCESS;
 }
 
+// ------------------------------------------- any two-factor length
+// K = r1 * r2, both register DFTs of at most MAXR points chosen at run time:
+// the block takes one branch of each phase, so a length costs no instance of
+// its own, and three register budgets (16, 24 and 32 points) cover the rest.
+// X[k1 + r1 k2] = sum_n2 W_r2^(n2 k2) W_K^(n2 k1) sum_n1 x[r2 n1 + n2] W_r1^(n1 k1).
+// What bounds the pass is memory; its data cross shared memory once (the
+// Stockham form: once a radix, with two buffers and index divisions per
+// butterfly, and 4 lines a block where the row is not a multiple of 16).
+// Measured, whole operator, Stockham -> this: forward 88 x 112 x 100 x 5 coils
+// (K 132, 168, 150) 1401 -> 907 us, adjoint 100 x 84 x 60 x 3 (200, 168, 120)
+// 459 -> 302 us, adjoint 256^2 x 8 (512) 110 -> 86 us.
+constexpr int kLines = 16;  // lines of a block: 128 contiguous bytes a point
+
+#define NUFFT_RADICES(X) \
+    X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16) \
+    X(18) X(20) X(21) X(22) X(24) X(25) X(26) X(27) X(28) X(30) X(32)
+
+template <int R>
+struct Radix {
+    static constexpr int value = R;
+};
+
+// calls f(Radix<r>())
+template <int MAXR, typename F>
+__device__ __forceinline__ void with_radix(int r, F &&f)
+{
+    switch (r) {
+#define NUFFT_CASE(R) case R: if constexpr (R <= MAXR) f(Radix<R>()); break;
+        NUFFT_RADICES(NUFFT_CASE)
+#undef NUFFT_CASE
+    default: break;
+    }
+}
+
+struct TwoStep {
+    int r1 = 0, r2 = 0, threads = 0;  // r1 <= r2; r1 = 0: no split
+};
+
+// The split with the smallest factors (fewest registers).  A thread takes one
+// r1-point column in turn (r2 / r1 rounds) and at most one r2-point row.
+static TwoStep two_step(int K)
+{
+    constexpr int radices[] = {
+#define NUFFT_LIST(R) R,
+        NUFFT_RADICES(NUFFT_LIST)
+#undef NUFFT_LIST
+    };
+    TwoStep t;
+    for (int r1 : radices)
+        for (int r2 : radices)
+            if (r1 <= r2 && r1 * r2 == K && (!t.r1 || r2 < t.r2)) {
+                t.r1 = r1;
+                t.r2 = r2;
+            }
+    if (t.r1) {
+        const int rounds = t.r2 / t.r1;
+        const int columns = (t.r2 + rounds - 1) / rounds;
+        t.threads = kLines * (columns > t.r1 ? columns : t.r1);
+    }
+    return t;
+}
+
+__host__ __device__ constexpr int two_step_pitch(int K) { return K | 1; }  // odd: no bank conflicts
+static size_t two_step_smem(int K) { return (size_t)(kLines * two_step_pitch(K) + K) * sizeof(float2); }
+
+constexpr int two_step_threads(int maxr) { return kLines * maxr; }
+constexpr int two_step_blocks(int maxr) { return maxr == 16 ? 4 : maxr == 24 ? 2 : 1; }
+
+// y or z pass; the last chunk of a row may be ragged.
+template <int MAXR>
+__global__ void __launch_bounds__(two_step_threads(MAXR), two_step_blocks(MAXR))
+k_line2(const float2 *__restrict__ in, float2 *__restrict__ out, LinePass lp, const float2 *__restrict__ twg,
+        int r1, int r2, int64_t rowlen, int inv)
+{
+    extern __shared__ float2 sm[];
+    const int K = r1 * r2, LS = two_step_pitch(K);
+    float2 *Y = sm;
+    float2 *tw = sm + kLines * LS;
+    for (int t = threadIdx.x; t < K; t += blockDim.x) tw[t] = twg[t];
+    const int outer = blockIdx.x / lp.nchunks;
+    const int64_t l0 = (int64_t)(blockIdx.x - outer * lp.nchunks) * kLines;
+    const int nl = (int)min((int64_t)kLines, rowlen - l0);
+    const float2 *ib = in + outer * lp.in_outer_stride + l0;
+    float2 *ob = out + outer * lp.out_outer_stride + l0;
+    const float sg = inv ? -1.f : 1.f;
+    const int Nh = lp.Nimg / 2, Nt = lp.Nimg - Nh;  // slot map as in line4_body
+    const int line = threadIdx.x % kLines;
+    const bool live = line < nl;
+    __syncthreads();
+    with_radix<MAXR>(r1, [&](auto radix) {
+        constexpr int R1 = decltype(radix)::value;
+        for (int n2 = threadIdx.x / kLines; n2 < r2; n2 += blockDim.x / kLines) {
+            float2 u[R1];
+#pragma unroll
+            for (int n1 = 0; n1 < R1; ++n1) {
+                const int pos = n2 + r2 * n1;
+                int src = pos;
+                if (lp.pad_in) src = pos < Nt ? pos + Nh : (pos >= K - Nh ? pos - (K - Nh) : -1);
+                float2 v = make_float2(0.f, 0.f);
+                if (live && src >= 0) {
+                    v = ib[(int64_t)src * lp.in_axis_stride + line];
+                    v.y *= sg;
+                }
+                u[n1] = v;
+            }
+            dft_reg<R1>(u);
+#pragma unroll
+            for (int k1 = 0; k1 < R1; ++k1) {
+                float2 x = u[k1];
+                if (k1) x = cmul(x, tw[n2 * k1]);
+                Y[line * LS + k1 * r2 + n2] = x;
+            }
+        }
+    });
+    __syncthreads();
+    const int k1 = threadIdx.x / kLines;
+    if (k1 >= r1 || !live) return;
+    with_radix<MAXR>(r2, [&](auto radix) {
+        constexpr int R2 = decltype(radix)::value;
+        float2 u[R2];
+#pragma unroll
+        for (int n2 = 0; n2 < R2; ++n2) u[n2] = Y[line * LS + k1 * R2 + n2];
+        dft_reg<R2>(u);
+#pragma unroll
+        for (int k2 = 0; k2 < R2; ++k2) {
+            const int k = k1 + r1 * k2;
+            int dst = k;
+            if (lp.crop_out) dst = k < Nt ? k + Nh : (k >= K - Nh ? k - (K - Nh) : -1);
+            if (dst >= 0) ob[(int64_t)dst * lp.out_axis_stride + line] = make_float2(u[k2].x, sg * u[k2].y);
+        }
+    });
+}
+
+// x pass; lines as in k_xline4.
+template <int MAXR, bool INV>
+__global__ void __launch_bounds__(two_step_threads(MAXR), two_step_blocks(MAXR))
+k_xline2(const float2 *__restrict__ in, float2 *__restrict__ out, const float *__restrict__ U,
+         const float2 *__restrict__ twg, int r1, int r2, int N1, int64_t N23, int nc, int64_t nlines, float scale,
+         const float2 *__restrict__ addend, float add_coef)
+{
+    extern __shared__ float2 sm[];
+    const int K = r1 * r2, LS = two_step_pitch(K);
+    float2 *Y = sm;
+    float2 *tw = sm + kLines * LS;
+    __shared__ int64_t rowb[kLines], intl[kLines], ub[kLines];  // as in k_xline4
+    for (int t = threadIdx.x; t < K; t += blockDim.x) tw[t] = twg[t];
+    if (threadIdx.x < kLines) {
+        const int64_t g = (int64_t)blockIdx.x * kLines + threadIdx.x;
+        const int64_t yz = g / nc;
+        const int c = (int)(g - yz * nc);
+        rowb[threadIdx.x] = ((int64_t)c * N23 + yz) * N1;
+        intl[threadIdx.x] = yz * K * nc + c;
+        ub[threadIdx.x] = g < nlines ? yz * N1 : -1;
+    }
+    const int Nh = N1 / 2, Nt = N1 - Nh;
+    __syncthreads();
+    with_radix<MAXR>(r1, [&](auto radix) {
+        constexpr int R1 = decltype(radix)::value;
+        for (int it = threadIdx.x; it < kLines * r2; it += blockDim.x) {
+            const int line = INV ? it % kLines : it / r2, n2 = INV ? it / kLines : it % r2;
+            const bool live = ub[line] >= 0;
+            float2 u[R1];
+#pragma unroll
+            for (int n1 = 0; n1 < R1; ++n1) {
+                const int pos = n2 + r2 * n1;
+                float2 v = make_float2(0.f, 0.f);
+                if (INV) {
+                    if (live) {
+                        v = in[intl[line] + (int64_t)pos * nc];
+                        v.y = -v.y;
+                    }
+                } else {
+                    const int src = pos < Nt ? pos + Nh : (pos >= K - Nh ? pos - (K - Nh) : -1);
+                    if (live && src >= 0) {
+                        const float2 x = in[rowb[line] + src];
+                        const float w = __ldg(&U[ub[line] + src]);
+                        v = make_float2(x.x * w, x.y * w);
+                    }
+                }
+                u[n1] = v;
+            }
+            dft_reg<R1>(u);
+#pragma unroll
+            for (int k1 = 0; k1 < R1; ++k1) {
+                float2 x = u[k1];
+                if (k1) x = cmul(x, tw[n2 * k1]);
+                Y[line * LS + k1 * r2 + n2] = x;
+            }
+        }
+    });
+    __syncthreads();
+    const int line = threadIdx.x % kLines, k1 = threadIdx.x / kLines;
+    const bool act = k1 < r1;
+    with_radix<MAXR>(r2, [&](auto radix) {
+        constexpr int R2 = decltype(radix)::value;
+        float2 u[R2];
+        if (act) {
+#pragma unroll
+            for (int n2 = 0; n2 < R2; ++n2) u[n2] = Y[line * LS + k1 * R2 + n2];
+            dft_reg<R2>(u);
+        }
+        if (INV) {
+            __syncthreads();  // every row has been read (the whole block takes this branch)
+            if (act) {
+#pragma unroll
+                for (int k2 = 0; k2 < R2; ++k2) Y[line * LS + k1 + r1 * k2] = u[k2];
+            }
+        } else if (act && ub[line] >= 0) {
+            float2 *ob = out + intl[line];
+#pragma unroll
+            for (int k2 = 0; k2 < R2; ++k2) ob[(int64_t)(k1 + r1 * k2) * nc] = u[k2];
+        }
+    });
+    if (!INV) return;
+    __syncthreads();
+    for (int it = threadIdx.x; it < kLines * N1; it += blockDim.x) {
+        const int ln = it / N1, n = it - ln * N1;
+        if (ub[ln] < 0) continue;
+        const float2 r = Y[ln * LS + slot_of(n, N1, K)];
+        const float w = __ldg(&U[ub[ln] + n]) * scale;
+        const int64_t idx = rowb[ln] + n;
+        float2 o = make_float2(r.x * w, -r.y * w);
+        if (addend) {
+            const float2 a = addend[idx];
+            o.x = fmaf(add_coef, a.x, o.x);
+            o.y = fmaf(add_coef, a.y, o.y);
+        }
+        out[idx] = o;
+    }
+}
+
+template <bool INV>
+static int launch_xline2(const TwoStep &t, const float2 *in, float2 *out, const float *U, const FFTDesc &fd, int N1,
+                         int64_t N23, int nc, float scale, const float2 *addend, float add_coef, cudaStream_t s)
+{
+    const int64_t nlines = N23 * nc;
+    const unsigned nblk = (unsigned)((nlines + kLines - 1) / kLines);
+    const size_t smem = two_step_smem(fd.n);
+    auto *k = t.r2 <= 16 ? k_xline2<16, INV> : t.r2 <= 24 ? k_xline2<24, INV> : k_xline2<32, INV>;
+    k<<<nblk, t.threads, smem, s>>>(in, out, U, fd.tw, t.r1, t.r2, N1, N23, nc, nlines, scale, addend, add_coef);
+    NUFFT_CUDA_TRY(cudaGetLastError());
+    return NUFFT3D_SUCCESS;
+}
+
+static int launch_line2(const TwoStep &t, const float2 *in, float2 *out, LinePass lp, const FFTDesc &fd,
+                        int n_outer, int64_t rowlen, int inv, cudaStream_t s)
+{
+    lp.nchunks = (int)((rowlen + kLines - 1) / kLines);
+    const int64_t nblk = (int64_t)n_outer * lp.nchunks;
+    auto *k = t.r2 <= 16 ? k_line2<16> : t.r2 <= 24 ? k_line2<24> : k_line2<32>;
+    k<<<(unsigned)nblk, t.threads, two_step_smem(fd.n), s>>>(in, out, lp, fd.tw, t.r1, t.r2, rowlen, inv);
+    NUFFT_CUDA_TRY(cudaGetLastError());
+    return NUFFT3D_SUCCESS;
+}
+
 int configure_fft_constants()
 {
-    auto fill = [](const void *sym, int n) {
-        std::vector<float2> w(n);
+    std::vector<float2> w(kMaxRadix * (kMaxRadix + 1) / 2);
+    for (int n = 1; n <= kMaxRadix; ++n)
         for (int j = 0; j < n; ++j) {
             const double a = -2.0 * M_PI * j / n;
-            w[j] = make_float2((float)std::cos(a), (float)std::sin(a));
+            w[n * (n - 1) / 2 + j] = make_float2((float)std::cos(a), (float)std::sin(a));
         }
-        return cudaMemcpyToSymbol(sym, w.data(), n * sizeof(float2));
-    };
-    NUFFT_CUDA_TRY(fill(c_w12, 12));
-    NUFFT_CUDA_TRY(fill(c_w16, 16));
-    NUFFT_CUDA_TRY(fill(c_w20, 20));
-    NUFFT_CUDA_TRY(fill(c_w24, 24));
+    NUFFT_CUDA_TRY(cudaMemcpyToSymbol(c_w, w.data(), w.size() * sizeof(float2)));
     return NUFFT3D_SUCCESS;
 }
 
@@ -706,6 +978,8 @@ static int launch_line(const float2 *in, float2 *out, int n_outer, int64_t rowle
     if (nblk > 0x7fffffff) return fail(NUFFT3D_ERR_SIZE, "FFT pass grid too large");
     const int r1 = four_step_r1(fd.n, lp.vec);
     if (r1) return launch_line4(r1, in, out, lp, fd, inv, nblk, s);
+    const TwoStep t = two_step(fd.n);
+    if (t.r1) return launch_line2(t, in, out, lp, fd, n_outer, rowlen, inv, s);
     if (needs_rare(fd))
         k_line<true><<<(unsigned)nblk, kFftThreads, line_smem(lp.vec, fd.n), s>>>(in, out, lp, fd, inv);
     else
@@ -787,6 +1061,8 @@ int launch_fx(nufft3d_plan *p, const float2 *img, float2 *B1, int nc, cudaStream
     const FFTDesc &fd = p->fft[0];
     if (const int r1 = four_step_r1(fd.n, 16))
         return launch_xline4<false>(r1, img, B1, p->U, fd, N1, N23, nc, 1.f, nullptr, 0.f, s);
+    const TwoStep t = two_step(fd.n);
+    if (t.r1) return launch_xline2<false>(t, img, B1, p->U, fd, N1, N23, nc, 1.f, nullptr, 0.f, s);
     const int nv = nc < kMaxLineCoils ? nc : kMaxLineCoils;
     dim3 grid(N23, (nc + kMaxLineCoils - 1) / kMaxLineCoils);
     if (needs_rare(fd))
@@ -804,6 +1080,8 @@ int launch_ix(nufft3d_plan *p, const float2 *B1, float2 *img, int nc, float scal
     const FFTDesc &fd = p->fft[0];
     if (const int r1 = four_step_r1(fd.n, 16))
         return launch_xline4<true>(r1, B1, img, p->U, fd, N1, N23, nc, scale, addend, add_coef, s);
+    const TwoStep t = two_step(fd.n);
+    if (t.r1) return launch_xline2<true>(t, B1, img, p->U, fd, N1, N23, nc, scale, addend, add_coef, s);
     const int nv = nc < kMaxLineCoils ? nc : kMaxLineCoils;
     dim3 grid(N23, (nc + kMaxLineCoils - 1) / kMaxLineCoils);
     if (needs_rare(fd))
@@ -830,8 +1108,9 @@ int launch_fz(nufft3d_plan *p, const float2 *B2, float2 *G, int nc, cudaStream_t
     const int64_t K1 = p->geom.K[0], K2 = p->geom.K[1], K3 = p->geom.K[2];
     const int64_t N3 = p->N[2];
     const int64_t row = K1 * nc;
-    return launch_line(B2, G, (int)K2, row, (int)N3, (int)K3, (int)N3, 1, 0, K2 * row, K2 * row,
-                       row, row, p->fft[2], 0, s);
+    // the rows of all y follow one another: one run of K2 * row lines
+    return launch_line(B2, G, 1, K2 * row, (int)N3, (int)K3, (int)N3, 1, 0, K2 * row, K2 * row,
+                       0, 0, p->fft[2], 0, s);
 }
 
 int launch_iz(nufft3d_plan *p, const float2 *G, float2 *B2, int nc, cudaStream_t s)
@@ -839,8 +1118,8 @@ int launch_iz(nufft3d_plan *p, const float2 *G, float2 *B2, int nc, cudaStream_t
     const int64_t K1 = p->geom.K[0], K2 = p->geom.K[1], K3 = p->geom.K[2];
     const int64_t N3 = p->N[2];
     const int64_t row = K1 * nc;
-    return launch_line(G, B2, (int)K2, row, (int)K3, (int)N3, (int)N3, 0, 1, K2 * row, K2 * row,
-                       row, row, p->fft[2], 1, s);
+    return launch_line(G, B2, 1, K2 * row, (int)K3, (int)N3, (int)N3, 0, 1, K2 * row, K2 * row,
+                       0, 0, p->fft[2], 1, s);
 }
 
 int launch_iy(nufft3d_plan *p, const float2 *B2, float2 *B1, int nc, cudaStream_t s)
@@ -894,6 +1173,15 @@ int configure_fft_kernels()
     NUFFT_TRY(allow_fft_smem(k_line4_batch_p<16>));
     NUFFT_TRY(allow_fft_smem(k_line4_batch_p<20>));
     NUFFT_TRY(allow_fft_smem(k_line4_batch_p<24>));
+    NUFFT_TRY(allow_fft_smem(k_line2<16>));
+    NUFFT_TRY(allow_fft_smem(k_xline2<16, false>));
+    NUFFT_TRY(allow_fft_smem(k_xline2<16, true>));
+    NUFFT_TRY(allow_fft_smem(k_line2<24>));
+    NUFFT_TRY(allow_fft_smem(k_xline2<24, false>));
+    NUFFT_TRY(allow_fft_smem(k_xline2<24, true>));
+    NUFFT_TRY(allow_fft_smem(k_line2<32>));
+    NUFFT_TRY(allow_fft_smem(k_xline2<32, false>));
+    NUFFT_TRY(allow_fft_smem(k_xline2<32, true>));
     return configure_fft_constants();
 }
 
