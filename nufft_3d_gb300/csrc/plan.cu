@@ -587,14 +587,16 @@ std::vector<int4> make_pieces(const std::vector<int32_t> &counts, int S)
     return blocks;
 }
 
-// Sign of image element i in the stored U: (-1)^(n - N/2) per transformed
-// axis (see grid_index).
-static int deap_sign(const nufft3d_plan *p, size_t i)
+// The signs of the stored U, applied or taken off: (-1)^(n - N/2) per
+// transformed axis (see grid_index).
+static void deap_signs(const nufft3d_plan *p, float *U)
 {
-    const size_t N1 = p->N[0], N2 = p->N[1];
-    size_t n = i % N1 + p->N[0] / 2 + i / N1 % N2 + p->N[1] / 2;
-    if (!p->geom.is2d) n += i / (N1 * N2) + p->N[2] / 2;
-    return n & 1 ? -1 : 1;
+    for (int z = 0; z < p->N[2]; ++z)
+        for (int y = 0; y < p->N[1]; ++y) {
+            const int row = p->N[0] / 2 + y + p->N[1] / 2 + (p->geom.is2d ? 0 : z + p->N[2] / 2);
+            float *u = U + ((size_t)z * p->N[1] + y) * p->N[0];
+            for (int x = row & 1 ? 0 : 1; x < p->N[0]; x += 2) u[x] = -u[x];
+        }
 }
 
 static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts &o)
@@ -737,7 +739,8 @@ static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts
     {
         std::vector<double> U = deap_host(p->N, g.K, p->J, p->alpha, g.radial, g.is2d);
         std::vector<float> Uf(U.size());
-        for (size_t i = 0; i < U.size(); ++i) Uf[i] = (float)U[i] * (float)deap_sign(p, i);
+        for (size_t i = 0; i < U.size(); ++i) Uf[i] = (float)U[i];
+        deap_signs(p, Uf.data());
         NUFFT_TRY(dmalloc(&p->U, Uf.size(), &p->table_bytes));
         NUFFT_CUDA_TRY(cudaMemcpyAsync(p->U, Uf.data(), sizeof(float) * Uf.size(), cudaMemcpyHostToDevice, s));
         NUFFT_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1140,7 +1143,7 @@ extern "C" int nufft3d_get_deap(const nufft3d_plan *p, float *U)
     DeviceGuard guard(p->device);
     const size_t n = (size_t)p->N[0] * p->N[1] * p->N[2];
     NUFFT_CUDA_TRY(cudaMemcpy(U, p->U, n * sizeof(float), cudaMemcpyDeviceToHost));
-    for (size_t i = 0; i < n; ++i) U[i] *= (float)deap_sign(p, i);
+    deap_signs(p, U);
     return NUFFT3D_SUCCESS;
 }
 
