@@ -114,7 +114,7 @@ def stage_bytes(obj, nc):
     """Algorithmic bytes per launch of each stage (reads + writes of its
     inputs/outputs).  Interpolation stages count the grid, the samples and
     12 bytes of coordinates per sample (per coil 8 K^3 + 8 M + 12 M/nc);
-    the stored H and H' that the 8-coil gather and spread read instead of
+    the stored H and H' that the gather and spread read instead of
     evaluating weights are reported beside them (`stored_h_bytes`,
     `stored_h_t_bytes`), not counted."""
     N1, N2, N3 = (int(v) for v in obj.N)
@@ -245,9 +245,7 @@ def bench_batched(maxit=20, damp=1e-3):
     import torch
     from nufft_3d_gb300 import NufftBatch, nufft_3d
     vols = uneven_volumes()
-    # the batched kernels read each volume's stored H but not its H' (the
-    # batched spread evaluates the kernel): plans made for a batch skip H'
-    objs = [nufft_3d(om, N, "J", 6, density_iters=20, spread_table=0) for om, N, _, _ in vols]
+    objs = [nufft_3d(om, N, "J", 6, density_iters=20) for om, N, _, _ in vols]
     ncs = [nc for _, _, nc, _ in vols]
     g = torch.Generator(device="cuda").manual_seed(0)
     raws = [torch.randn((nc, o.M), dtype=torch.complex64, device="cuda", generator=g) for o, nc in zip(objs, ncs)]
@@ -483,7 +481,7 @@ def main():
     ap.add_argument("--e2e-free-sms", dest="e2e_free_sms", type=int, default=None,
                     help="e2e leg: multiprocessors the handles' interpolation kernels leave free")
     ap.add_argument("--spread-table", dest="spread_table", type=int, default=-1, choices=[-1, 0, 1],
-                    help="stored H' for the 8-coil spread: -1 auto (library default), 0 on the fly, 1 always")
+                    help="stored H' for the spread: -1 auto (library default), 0 on the fly, 1 always")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
     if args.impl == "reference":

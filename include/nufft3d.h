@@ -65,7 +65,7 @@ typedef struct nufft3d_opts {
     int max_samples_per_block; /* samples per interpolation block (0 = 4096) */
     int verbose;       /* print the reference's set-up summary to stdout */
     int tap_table;     /* stored interpolation matrix H (nufft_3d.m:153-212) in
-                          tile order, read by the 8-coil gather passes of fNUFT
+                          tile order, read by the gather passes of fNUFT
                           (see spread_table for H'): 1 = build it, 0 = evaluate
                           the kernel on the fly, -1 = auto (default: build it
                           when it takes at most half of the free device memory) */
@@ -76,11 +76,11 @@ typedef struct nufft3d_opts {
                           copy is then still allowed to land, but its tile is
                           skipped and the timeout reported, which exercises the
                           error path without a fault */
-    int spread_table;  /* stored transpose H' (built from the stored H, so only
-                          with it), read by the 8-coil spread passes of aNUFT
-                          (full passes of an even coil count): per tile piece
-                          of at most 2048 samples, each grid point's row of
-                          (sample, weight); 1 = build it, 0 = evaluate the
+    int spread_table;  /* stored transpose H' (only beside the stored H), read by
+                          the spread passes of aNUFT (passes of fewer than 8
+                          coils: from 32768 samples on): per piece of at most
+                          1664 samples, rows of 2 x 2 grid points, a sample and
+                          four weights an entry; 1 = build it, 0 = evaluate the
                           kernel on the fly, -1 = auto (default: build it when
                           it takes at most half of the free device memory) */
 } nufft3d_opts;
@@ -256,9 +256,8 @@ int nufft3d_inverse_x0_host(nufft3d_plan *plan, const float *raw_host, float *x_
  * gives.  plans[v] must be distinct handles (nufft3d_plan_share for repeated
  * trajectories) sharing the kernel (J, u, alpha, radial) and 2-D/3-D; the batch
  * uses their work buffers, so do not use those handles concurrently with it.
- * The batched kernels read each volume's stored H (tap_table) but not its
- * stored H' (the batched spread evaluates the kernel): plans made only for
- * batches can set spread_table = 0 and save that memory. */
+ * The batch reads the stored H (tap_table) and the stored H' (spread_table)
+ * when every volume has it, and otherwise evaluates the kernel for all. */
 typedef struct nufft3d_batch nufft3d_batch;
 int nufft3d_batch_create(nufft3d_plan *const *plans, const int *nc, int nvol, nufft3d_batch **batch);
 int nufft3d_batch_destroy(nufft3d_batch *batch);

@@ -96,7 +96,7 @@ class nufft_3d:  # noqa: N801  (the reference's class name)
             opts.tap_table = int(tap_table)
         if wait_polls is not None:  # polls of each bounded wait (0: give up at once)
             opts.wait_polls = int(wait_polls)
-        if spread_table is not None:  # stored H' for the 8-coil spread: 1 build, 0 on the fly, -1 auto
+        if spread_table is not None:  # stored H' for the spread: 1 build, 0 on the fly, -1 auto
             opts.spread_table = int(spread_table)
         dbuf = None
         if pairs.get("d") is not None:
