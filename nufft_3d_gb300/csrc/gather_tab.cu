@@ -197,35 +197,42 @@ __device__ __forceinline__ void copy_pairs(const GatherArgs &a, const uint32_t *
 
 // ... and coil counts whose points are not whole 16-byte units coil by coil,
 // through registers, several loads in flight (8-byte asynchronous copies took
-// three times as long).
-template <int CB>
+// three times as long).  A warp takes whole points, 32 at a time, so that it
+// reads only the offsets that it wrote, whatever the coil count (5 coils on
+// 88 x 112 x 100: forward 747 us, indices found by division a coil 857 us).
+template <int CB, int NPW>
 __device__ __forceinline__ void copy_coils(const GatherArgs &a, const uint32_t *poff, unsigned char *ring,
-                                           unsigned pbytes, int slot, int z0, int n, int t, int nt)
+                                           unsigned pbytes, int slot, int z0, int n, int pw, int lane)
 {
-    const int ne = a.P0 * a.P1 * CB, per = (ne + nt - 1) / nt;  // coils of a plane, of a thread in a plane
-    constexpr int U = CB >= 3 ? 16 : 8;
-    int k = 0, p = 0;
+    constexpr int M = CB >= 7 ? 2 : CB == 5 ? 3 : CB == 3 ? 5 : CB == 1 ? 8 : 4;  // groups of 32 points in flight
+    const int npt = a.P0 * a.P1;
+    const int per = (npt + 32 * NPW - 1) / (32 * NPW);  // groups of a warp in a plane
+    int i = 0, p = 0;
     size_t plane = grid_plane(a, z0);
     while (p < n) {
-        float2 v[U];
-        unsigned d[U];
+        float2 v[M * CB];
+        unsigned d[M * CB];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int e = t + k * nt, pt = e / CB, c = e - pt * CB;
-            d[u] = 0xffffffffu;
-            if (p < n && e < ne && c < a.cb) {
-                v[u] = __ldcg(a.G + (plane + poff[pt]) * a.nc + a.c0 + c);
-                d[u] = (unsigned)slot * pbytes + 8u * e;
+        for (int m = 0; m < M; ++m) {
+            const int pt0 = (pw + NPW * i) * 32;
+#pragma unroll
+            for (int j = 0; j < CB; ++j) {
+                const int e = j * 32 + lane, pt = pt0 + e / CB, c = e % CB;
+                d[m * CB + j] = 0xffffffffu;
+                if (p < n && pt < npt && c < a.cb) {
+                    v[m * CB + j] = __ldcg(a.G + (plane + poff[pt]) * a.nc + a.c0 + c);
+                    d[m * CB + j] = (unsigned)slot * pbytes + 8u * (unsigned)(pt0 * CB + e);
+                }
             }
-            if (++k == per) {
-                k = 0;
+            if (++i == per) {
+                i = 0;
                 ++p;
                 if (++slot == a.S) slot = 0;
                 plane = grid_plane(a, z0 + p);
             }
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < M * CB; ++u)
             if (d[u] != 0xffffffffu) *reinterpret_cast<float2 *>(ring + d[u]) = v[u];
     }
 }
@@ -428,13 +435,13 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
                         col_y = rec.oy;
                         __syncwarp();
                         if (pairs) plane_offsets<kUnits<CB>>(a, poff, col_x, col_y, t, 32 * NPW);
-                        else plane_offsets<CB>(a, poff, col_x, col_y, t, 32 * NPW);
+                        else plane_offsets<1>(a, poff, col_x, col_y, t, 32 * NPW);
                         __syncwarp();
                     }
                     if constexpr (kPaired<CB>) {
                         if (pairs) copy_pairs<CB>(a, poff, ring, pbytes, slot, z0, rec.nload, t, 32 * NPW);
                     }
-                    if (!pairs) copy_coils<CB>(a, poff, gsm, pbytes, slot, z0, rec.nload, t, 32 * NPW);
+                    if (!pairs) copy_coils<CB, NPW>(a, poff, gsm, pbytes, slot, z0, rec.nload, pw, lane);
                 }
                 endp += rec.nload;
                 slot += rec.nload;
@@ -861,15 +868,16 @@ static void make_records(const nufft3d_plan *p, std::vector<GatherRec> &recs, ui
 }
 
 // Record ranges: each about a sixth of what is left for each multiprocessor
-// (rows, a loaded plane counting as four, or 16 where the tile wraps around
-// the grid edge and is copied piecemeal), so that the last ones are short,
+// (rows, a loaded plane of 14 x 14 points counting as four, or 16 where the
+// tile wraps around the grid edge and is copied piecemeal), so that the last ones are short,
 // and at least 128 rows, below which the planes that a range loads anew
 // outweigh its rows.
 static std::vector<int2> make_chunks(const std::vector<GatherRec> &recs, const Geom &g, int sms)
 {
+    const int plane = std::max(1, plane_stride(g) / 196);  // planes of 14 x 14 points
     auto cost = [&](const GatherRec &r) {
         const bool inside = r.ox >= 0 && r.oy >= 0 && r.ox + g.P[0] <= g.K[0] && r.oy + g.P[1] <= g.K[1];
-        return r.nrows + (inside ? 4 : 16) * r.nload;
+        return r.nrows + (inside ? 4 : 16) * r.nload * plane;
     };
     int64_t left = 0;
     for (auto &r : recs) left += cost(r);
@@ -1040,15 +1048,26 @@ int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int 
     const bool odd = nc == a.cb && nc % 2 == 1 && nc < 8;
     if (odd) cb = nc;
     a.use_tma = p->use_tma && encode_plane_map(p, G, nc, cb, &m) ? 1 : 0;
+    // Tiles that wrap around the grid edge are copied by the producer warps, not
+    // by bulk copies.  Four of them instead of one where such tiles are common
+    // (percentage of inner tiles below the limit) gain on the copies what the
+    // consumers lose in warps, the more the wider the pass: forward of 8 coils
+    // at 32^3 (56 % inner, 16384 random samples) 98 -> 76 us, 7 coils at
+    // 88 x 112 x 100 (79 %, 1000003) 2177 -> 1509 us, 5 coils at 128^3 (87 %)
+    // 1922 -> 1734 us; past the limits one is better: 4 coils at 128^3 1568 ->
+    // 1401 us, one coil at 64^3 (76 %, 262144) 155 -> 111 us.  A 2-D plane is a
+    // whole tile of 38 x 38 points (324 x 98, 3 coils: 166 -> 58 us, with the
+    // shorter ranges of make_chunks).
+    const int inner = 100 * std::max(0, g.nt[0] - 2) * std::max(0, g.nt[1] - 2) / (g.nt[0] * g.nt[1]);
+    const bool copies = !a.use_tma || g.is2d || inner < (cb <= 2 ? 50 : cb % 2 == 0 ? 79 : cb == 3 ? 85 : 90);
     switch (cb) {
-    case 1: return launch_rows<1, 1>(p, a, m, s);
-    case 2: return launch_rows<2, 1>(p, a, m, s);
-    case 3: return launch_rows<3, 1>(p, a, m, s);
-    case 5: return launch_rows<5, 1>(p, a, m, s);
-    case 7: return launch_rows<7, 1>(p, a, m, s);
-    // without bulk copies four producer warps keep up with the consumers
-    case 4: return a.use_tma ? launch_rows<4, 1>(p, a, m, s) : launch_rows<4, 4>(p, a, m, s);
-    default: return a.use_tma ? launch_rows<8, 1>(p, a, m, s) : launch_rows<8, 4>(p, a, m, s);
+    case 1: return copies ? launch_rows<1, 4>(p, a, m, s) : launch_rows<1, 1>(p, a, m, s);
+    case 2: return copies ? launch_rows<2, 4>(p, a, m, s) : launch_rows<2, 1>(p, a, m, s);
+    case 3: return copies ? launch_rows<3, 4>(p, a, m, s) : launch_rows<3, 1>(p, a, m, s);
+    case 5: return copies ? launch_rows<5, 4>(p, a, m, s) : launch_rows<5, 1>(p, a, m, s);
+    case 7: return copies ? launch_rows<7, 4>(p, a, m, s) : launch_rows<7, 1>(p, a, m, s);
+    case 4: return copies ? launch_rows<4, 4>(p, a, m, s) : launch_rows<4, 1>(p, a, m, s);
+    default: return copies ? launch_rows<8, 4>(p, a, m, s) : launch_rows<8, 1>(p, a, m, s);
     }
 }
 
@@ -1065,10 +1084,15 @@ static int allow_rows()
 int configure_gather_tab_kernels()
 {
     NUFFT_TRY((allow_rows<1, 1>()));
+    NUFFT_TRY((allow_rows<1, 4>()));
     NUFFT_TRY((allow_rows<2, 1>()));
+    NUFFT_TRY((allow_rows<2, 4>()));
     NUFFT_TRY((allow_rows<3, 1>()));
+    NUFFT_TRY((allow_rows<3, 4>()));
     NUFFT_TRY((allow_rows<5, 1>()));
+    NUFFT_TRY((allow_rows<5, 4>()));
     NUFFT_TRY((allow_rows<7, 1>()));
+    NUFFT_TRY((allow_rows<7, 4>()));
     NUFFT_TRY((allow_rows<4, 1>()));
     NUFFT_TRY((allow_rows<4, 4>()));
     NUFFT_TRY((allow_rows<8, 1>()));

@@ -74,3 +74,11 @@ def test_samples_of_a_slab(counts, nc):
         centre = np.array([3.0 - 5 * i, -2.0, 1.0]) if i + 1 < len(counts) or len(counts) == 1 else np.array([7.2, 7.5, -7.7])
         pts.append(centre[:, None] + rng.uniform(-0.2, 0.2, (3, c)))
     _case(16, np.concatenate(pts, axis=1), nc, dict(J=6, u=2))
+
+
+@pytest.mark.parametrize("nc", [1, 2, 3, 4, 5, 6, 7, 8])
+def test_one_producer(nc):
+    """A grid of 40 x 40 tiles a plane, nine tenths of them inside: bulk copies by a single warp at every width."""
+    rng = np.random.default_rng(nc)
+    om = np.stack([rng.uniform(-n / 2, n / 2 - 1, 20000) for n in (160, 160, 6)])
+    _case((160, 160, 6), om, nc, dict(J=6, u=2))
