@@ -63,6 +63,7 @@
 #include "async.h"
 #include "internal.h"
 #include "taps.h"
+#include "waits.h"
 
 namespace nufft3d {
 
@@ -270,15 +271,36 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
     }
     __syncthreads();
     const unsigned pbytes = (unsigned)a.PS * SLOT;
+    // A wait that runs out is reported and ends the block's work.  A warp takes
+    // that decision as one (lane 0 waits and tells the others, or they vote): a
+    // lane that left alone would leave the others at the next warp-wide
+    // instruction.
     volatile int *const ab = &ctl[3];
+    auto give_up = [&]() {
+        if (lane == 0) {
+            if (a.st.err) atomicOr(a.st.err, 1);
+            *ab = 1;
+        }
+    };
+    auto ended = [&]() { return __any_sync(0xffffffffu, *ab != 0) != 0; };
+    // records issued by the first producer warp, once it has stopped (-1: it has not)
+    auto records = [&]() {
+        for (int i = 0; i < kDrainPolls; ++i) {
+            const int n = __reduce_min_sync(0xffffffffu, ld_acquire(&nrec[1]));
+            if (n != 0x7fffffff) return n;
+            __nanosleep(50);
+        }
+        return -1;
+    };
 
     if (warp >= NW + NPW) {
         // ---------------------------------------------------------- helper
         // Publishes the tasks of each record once its planes and those of the
         // records before it (it shares planes with them) have landed.
-        int ahead = 0, landed = 0, tries = 0;
+        int ahead = 0, landed = 0;
+        BoundedWait copy, idle;
         for (;;) {
-            const int n = ld_acquire(&nrec[0]);
+            const int n = __reduce_min_sync(0xffffffffu, ld_acquire(&nrec[0]));
             if (ahead < n) {
                 if (kPrefetch<CB> && n - ahead < kStages) {  // (else the slot may be in new use)
                     const uint2 q = ahead_of[ahead % kStages];
@@ -288,31 +310,40 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
                     for (unsigned o = 128u * lane; o < 32u * q.y; o += 128u * 32) prefetch_line(x + o);
                 }
                 ++ahead;
+                idle = BoundedWait();
                 continue;
             }
             if (landed < n) {
                 const int st = landed % kStages;
-                const bool late = tries++ == a.st.polls;
-                if (late && lane == 0 && a.st.err) atomicOr(a.st.err, 1);  // expired: reported, and waited for all the same
-                if (mbar_try_wait(full + 8 * st, (unsigned)(landed / kStages) & 1u)) {
-                    __syncwarp();
+                const WaitTurn turn = wait_turn(copy, a.st.polls, kDrainPolls);
+                // expired: reported, and waited for all the same
+                if (turn == kWaitReport && lane == 0 && a.st.err) atomicOr(a.st.err, 1);
+                if (turn == kWaitGiveUp) {
+                    give_up();
+                } else if (__all_sync(0xffffffffu, mbar_try_wait(full + 8 * st, (unsigned)(landed / kStages) & 1u))) {
                     if (lane == 0) st_release(&ctl[0], tend[st]);
                     ++landed;
-                    tries = 0;
-                } else if (tries >= kDrainPolls) {
-                    *ab = 1;
+                    copy = BoundedWait();
+                } else {
+                    ++copy.failed;
                 }
-            } else if (ld_acquire(&nrec[1]) <= landed) {
+            } else if (__all_sync(0xffffffffu, ld_acquire(&nrec[1]) <= landed)) {
                 break;
             } else {
-                if (++tries >= kDrainPolls) {
-                    if (lane == 0 && a.st.err) atomicOr(a.st.err, 1);
-                    *ab = 1;
-                }
+                if (wait_turn(idle, kDrainPolls, kDrainPolls) == kWaitGiveUp) give_up();
+                ++idle.failed;
                 __nanosleep(50);
-                if (ld_acquire(&nrec[0]) > landed) tries = 0;
             }
-            if (*ab) break;
+            if (ended()) break;
+        }
+        if (ended()) {
+            // the block must not leave while planes are on their way to its memory
+            const int n = records();
+            for (; landed < n; ++landed)
+                for (int i = 0; i < kDrainPolls; ++i)
+                    if (__all_sync(0xffffffffu, mbar_try_wait(full + 8 * (landed % kStages),
+                                                              (unsigned)(landed / kStages) & 1u)))
+                        break;
         }
     } else if (warp >= NW) {
         // ------------------------------------------------------ producers
@@ -389,21 +420,23 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
             rows += rec.nrows;
             while (d < rr && (rr - d >= kStages || send[d % kStages] - a.npl < endp + rec.nload - a.S ||
                               rows - srow[d % kStages] > kRowsAhead)) {
-                const int want = stask[d % kStages];
-                bool ok = false;
-                for (int t = 0; t < kDrainPolls && !ok && !*ab; ++t) {
-                    ok = ld_acquire(&finished[d % kStages]) - want >= 0;
-                    if (!ok) __nanosleep(50);
+                int ok = 0;
+                if (lane == 0) {
+                    const int want = stask[d % kStages];
+                    for (int t = 0; t < kDrainPolls && !ok && !*ab; ++t) {
+                        ok = ld_acquire(&finished[d % kStages]) - want >= 0;
+                        if (!ok) __nanosleep(50);
+                    }
                 }
-                if (!ok) {
-                    if (a.st.err) atomicOr(a.st.err, 1);
-                    *ab = 1;
+                if (!__shfl_sync(0xffffffffu, ok, 0)) {
+                    give_up();
                     live = false;
                     break;
                 }
                 ++d;
             }
             if (!live) break;
+            __syncwarp();  // what lane 0 saw finished is finished for every lane
             const int st = rr % kStages;
             const unsigned fb = full + 8 * st;
             const bool pairs = kPaired<CB> && a.pairs;
@@ -484,6 +517,10 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
             st_release(&ctl[2], ntasks);
             st_release(&nrec[1], rr);
         }
+        // the helper waits for the planes of every record issued: without this
+        // warp's arrivals it would not see them land
+        if (!live && pw > 0)
+            for (const int n = records(); rr < n; ++rr) mbar_arrive(full + 8 * (rr % kStages));
         // no exit before this thread's copies have landed
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
@@ -505,21 +542,21 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
         int task = lane == 0 ? atomicAdd(&ctl[1], 1) : 0;
         // Starts the loads of the warp's next task; false at the end.
         auto next_task = [&]() -> bool {
-            const int t = __shfl_sync(0xffffffffu, task, 0);
-            if (lane == 0) task = atomicAdd(&ctl[1], 1);
-            bool ok = false, end = false;
-            for (int i = 0; i < kDrainPolls && !ok && !end; ++i) {
-                ok = ld_acquire(&ctl[0]) > t;
-                end = !ok && (ld_acquire(&ctl[2]) <= t || *ab);
-                if (!ok) __nanosleep(50);
-            }
-            if (!ok) {
-                if (!end) {  // expired
-                    if (lane == 0 && a.st.err) atomicOr(a.st.err, 1);
-                    *ab = 1;
+            int t = -2;  // expired, -1: no more tasks
+            if (lane == 0) {
+                for (int i = 0; i < kDrainPolls && t == -2; ++i) {
+                    if (ld_acquire(&ctl[0]) > task) t = task;
+                    else if (ld_acquire(&ctl[2]) <= task || *ab) t = -1;
+                    else __nanosleep(50);
                 }
+                task = atomicAdd(&ctl[1], 1);
+            }
+            t = __shfl_sync(0xffffffffu, t, 0);
+            if (t < 0) {
+                if (t == -2) give_up();
                 return false;
             }
+            __syncwarp();  // what lane 0 saw published is seen by every lane
             const GatherTask &f = tasks[t % kTasks];
             const int4 g = *reinterpret_cast<const int4 *>(&f);
             stage = g.w;
