@@ -937,21 +937,29 @@ bool fft_factor(int n, FFTDesc &d)
     return m == 1;
 }
 
-int line_vec(int64_t rowlen)
+size_t line_smem(int vec, int K) { return (size_t)2 * vec * (K + 1) * sizeof(float2); }
+
+// Lines of a block of a y or z pass of length K.  The Stockham form holds two
+// buffers of them in shared memory: 16 lines of 908 points do not fit, and
+// fewer leave room for more blocks, down to 4 lines (one 32-byte sector a
+// point).  z passes in us at the 16 or 8 lines that fit, at 4 lines: K = 490,
+// 8 coils on 128 x 128 rows 1207, 635 (inverse 1597, 669); K = 686, one coil on
+// 120 x 120 163, 101; K = 1000, one coil on 100 x 100 187, 107.
+constexpr size_t kStockhamSmem = 40 * 1024;
+
+int line_vec(int64_t rowlen, int K)
 {
     const int cands[] = {16, 8, 4, 2, 1};
     for (int v : cands)
-        if (rowlen % v == 0) return v;
+        if (rowlen % v == 0 && (v <= 4 || four_step_r1(K, v) || line_smem(v, K) <= kStockhamSmem)) return v;
     return 1;
 }
-
-size_t line_smem(int vec, int K) { return (size_t)2 * vec * (K + 1) * sizeof(float2); }
 
 LinePass make_linepass(int n_outer, int64_t rowlen, int n_in, int n_out, int Nimg, int pad_in, int crop_out,
                        int64_t in_axis, int64_t out_axis, int64_t in_outer, int64_t out_outer, int64_t *nblk)
 {
     LinePass lp;
-    lp.vec = line_vec(rowlen);
+    lp.vec = line_vec(rowlen, n_in > n_out ? n_in : n_out);
     lp.nchunks = (int)(rowlen / lp.vec);
     lp.n_in = n_in;
     lp.n_out = n_out;

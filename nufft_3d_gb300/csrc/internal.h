@@ -231,7 +231,7 @@ struct BatchPerm {
 
 LinePass make_linepass(int n_outer, int64_t rowlen, int n_in, int n_out, int Nimg, int pad_in, int crop_out,
                        int64_t in_axis, int64_t out_axis, int64_t in_outer, int64_t out_outer, int64_t *nblk);
-int line_vec(int64_t rowlen);
+int line_vec(int64_t rowlen, int K);
 size_t line_smem(int vec, int K);
 bool needs_rare(const FFTDesc &f);
 constexpr int kMaxLineCoilsHost = 16;

@@ -56,3 +56,25 @@ def test_other_oversampling(N, u, nc):
     fr = ref.fNUFT(x)
     f = f.reshape(nc, -1).T
     assert np.linalg.norm(f - fr.reshape(f.shape)) < 1e-5 * np.linalg.norm(fr)
+
+
+@pytest.mark.parametrize("N,u,nc", [((10, 6, 500), 2, 1), ((6, 8, 500), 2, 3), ((6, 500, 8), 2, 4),
+                                    ((8, 6, 454), 910 / 454 - 1e-9, 1), ((6, 6, 528), 2, 2)])
+def test_long_lengths_without_a_split(N, u, nc):
+    """K = 1000, 910, 1056 on the y and z axes: 16 lines of two Stockham buffers would not fit in shared memory."""
+    import torch
+
+    from nufft_3d_gb300 import nufft_3d
+    rng = np.random.default_rng(N[2])
+    om = np.stack([rng.uniform(-n / 2, n / 2 - 1, 1500) for n in N])
+    obj = nufft_3d(om, N, J=4, u=u, density_iters=0)
+    ref = NufftRef(om, N, J=4, u=u, density_iters=0)
+    x = rng.standard_normal((*N, nc)) + 1j * rng.standard_normal((*N, nc))
+    y = rng.standard_normal((1500, nc)) + 1j * rng.standard_normal((1500, nc))
+    f = obj.fNUFT(torch.from_numpy(x.transpose(3, 2, 1, 0).astype(np.complex64)).cuda()).cpu().numpy()
+    a = obj.aNUFT(torch.from_numpy(np.ascontiguousarray(y.T).astype(np.complex64)).cuda()).cpu().numpy()
+    fr, ar = ref.fNUFT(x), ref.aNUFT(y)
+    f = f.reshape(nc, -1).T
+    a = a.transpose(3, 2, 1, 0)
+    assert np.linalg.norm(f - fr.reshape(f.shape)) < 1e-5 * np.linalg.norm(fr)
+    assert np.linalg.norm(a - ar.reshape(a.shape)) < 1e-5 * np.linalg.norm(ar)
