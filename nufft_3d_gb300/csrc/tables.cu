@@ -618,7 +618,12 @@ k_spread_rows(const float2 *__restrict__ ks, float2 *__restrict__ G, int nc, int
                 }
             }
         };
-        auto line = [&](const float4 w, unsigned sx) {
+        // A step's lines are summed by themselves: a quarter of the additions to
+        // the long sums, whose rounding grows with their number (64^3 koosh
+        // ball, 8 coils: error against FP64 1.29e-7 -> 1.23e-7, the time as before).
+        float2 sum4[NQ][NU * NV];
+        auto line = [&](const float4 w, unsigned sx, bool first) {
+            auto mad = [&](float2 x, float2 y, float2 c) { return first ? __fmul2_rn(x, y) : __ffma2_rn(x, y, c); };
             const unsigned char *y = ys + sx * SLOT;
             const float ws[4] = {w.x, w.y, w.z, w.w};
             if constexpr (CB >= 4) {
@@ -630,22 +635,22 @@ k_spread_rows(const float2 *__restrict__ ks, float2 *__restrict__ G, int nc, int
                     const float2 ww = make_float2(ws[q], ws[q]);
 #pragma unroll
                     for (int k = 0; k < NU; ++k) {
-                        acc[q][2 * k] = __ffma2_rn(ww, make_float2(v[k].x, v[k].y), acc[q][2 * k]);
-                        acc[q][2 * k + 1] = __ffma2_rn(ww, make_float2(v[k].z, v[k].w), acc[q][2 * k + 1]);
+                        sum4[q][2 * k] = mad(ww, make_float2(v[k].x, v[k].y), sum4[q][2 * k]);
+                        sum4[q][2 * k + 1] = mad(ww, make_float2(v[k].z, v[k].w), sum4[q][2 * k + 1]);
                     }
                 }
             } else {
                 const float wa = h ? w.y : w.x, wb = h ? w.w : w.z;
                 if constexpr (CB == 2) {
                     const float4 v = *reinterpret_cast<const float4 *>(y);
-                    acc[0][0] = __ffma2_rn(make_float2(wa, wa), make_float2(v.x, v.y), acc[0][0]);
-                    acc[0][1] = __ffma2_rn(make_float2(wa, wa), make_float2(v.z, v.w), acc[0][1]);
-                    acc[1][0] = __ffma2_rn(make_float2(wb, wb), make_float2(v.x, v.y), acc[1][0]);
-                    acc[1][1] = __ffma2_rn(make_float2(wb, wb), make_float2(v.z, v.w), acc[1][1]);
+                    sum4[0][0] = mad(make_float2(wa, wa), make_float2(v.x, v.y), sum4[0][0]);
+                    sum4[0][1] = mad(make_float2(wa, wa), make_float2(v.z, v.w), sum4[0][1]);
+                    sum4[1][0] = mad(make_float2(wb, wb), make_float2(v.x, v.y), sum4[1][0]);
+                    sum4[1][1] = mad(make_float2(wb, wb), make_float2(v.z, v.w), sum4[1][1]);
                 } else {
                     const float2 v = *reinterpret_cast<const float2 *>(y);
-                    acc[0][0] = __ffma2_rn(make_float2(wa, wa), v, acc[0][0]);
-                    acc[1][0] = __ffma2_rn(make_float2(wb, wb), v, acc[1][0]);
+                    sum4[0][0] = mad(make_float2(wa, wa), v, sum4[0][0]);
+                    sum4[1][0] = mad(make_float2(wb, wb), v, sum4[1][0]);
                 }
             }
         };
@@ -665,8 +670,12 @@ k_spread_rows(const float2 *__restrict__ ks, float2 *__restrict__ G, int nc, int
                     const unsigned sx = x[k];
                     e[k] = ld_stream4(lw + (size_t)(l + k + D) * kRows);
                     x[k] = ld_stream16(lx + (size_t)(l + k + D) * kRows);
-                    line(w, sx);
+                    line(w, sx, k == 0);
                 }
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+#pragma unroll
+                    for (int c = 0; c < NU * NV; ++c) acc[q][c] = __fadd2_rn(acc[q][c], sum4[q][c]);
             }
             add_points();
             clear();
@@ -744,7 +753,11 @@ int configure_spread_tab_kernels()
 
 // Pieces of at most cap samples: runs of slabs of one column, or shares of a
 // larger slab; most samples first (the heavy centre of radial k-space starts
-// early).  ext: slabs of each piece.
+// early).  ext: slabs of each piece.  A larger slab is dealt to pieces of up to
+// kSpreadCap whatever cap is: every one of them adds to the same few points of
+// the grid, and the rounding of those sums grows with their number (64^3 koosh
+// ball, 8 coils, shares of 431 samples: error against FP64 2.2e-7, of 1664
+// 1.3e-7; one coil 124 and 129 us).
 static void make_spread_pieces(const nufft3d_plan *p, int cap, std::vector<int4> &pcs, std::vector<int> &ext)
 {
     const Geom &g = p->geom;
@@ -767,7 +780,7 @@ static void make_spread_pieces(const nufft3d_plan *p, int cap, std::vector<int4>
         if (c == 0) continue;
         if (start >= 0 && (i / col_slabs != start / col_slabs || i - start >= max_slabs || count + c > cap)) close(last + 1);
         if (c > cap) {
-            const int nb = (c + cap - 1) / cap;
+            const int nb = (c + kSpreadCap - 1) / kSpreadCap;
             for (int b = 0; b < nb; ++b)
                 runs.push_back({make_int4((int)(off + b), (c - b + nb - 1) / nb | nb << kCountBits, 0, i), 1});
         } else {
@@ -801,8 +814,8 @@ int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s)
 {
     if (mode == 0 || p->gw == nullptr || p->nnz == 0) return NUFFT3D_SUCCESS;
     const Geom &g = p->geom;
-    // About four pieces a multiprocessor where the samples are few (64^3 x 1 coil,
-    // 262144 samples: 80 us, with the largest pieces 99 us).  A 2-D piece holds
+    // Runs for about four pieces a multiprocessor where the samples are few (64^3
+    // x 1 coil, 262144 samples: 85 us, with the largest pieces 99 us).  A 2-D piece holds
     // a whole tile of 38 x 38 points however few its samples are, so there
     // smaller pieces only add points (256^2 x 8 coils: 27 us, four a
     // multiprocessor 41 us).
@@ -904,7 +917,8 @@ int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s)
     p->spread_pieces = pieces;
     p->spread_wstart = wst;
     p->n_spread_pieces = np;
-    p->spread_cap = cap;
+    p->spread_cap = 0;
+    for (auto &pc : pcs) p->spread_cap = std::max(p->spread_cap, piece_count(pc));
     p->spread_bytes = (int64_t)(bytes + wbytes + sizeof(int4) * np);
     p->table_bytes += p->spread_bytes;
     keep.ptrs.clear();
