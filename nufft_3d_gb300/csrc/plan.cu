@@ -731,8 +731,8 @@ static int build_plan(nufft3d_plan *p, const double *om_host, const nufft3d_opts
             p->cand_desc.core[q] = cs.core[q];
         }
     }
-    NUFFT_TRY(launch_weight_sum(p, s));
     NUFFT_TRY(build_gather_table(p, o.tap_table, s));
+    NUFFT_TRY(launch_weight_sum(p, s));  // (the stored H moves samples between the pieces)
     NUFFT_TRY(build_spread_table(p, o.spread_table, s));
     std::vector<int32_t>().swap(p->slab_counts);
     // deapodization (FP64 on the host, stored FP32 like deap.m:100-101)

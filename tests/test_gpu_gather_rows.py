@@ -82,3 +82,22 @@ def test_one_producer(nc):
     rng = np.random.default_rng(nc)
     om = np.stack([rng.uniform(-n / 2, n / 2 - 1, 20000) for n in (160, 160, 6)])
     _case((160, 160, 6), om, nc, dict(J=6, u=2))
+
+
+@pytest.mark.parametrize("nc", [1, 8])
+def test_rows_move_samples_between_small_pieces(nc):
+    """Pieces of 64 samples, half a record of the stored H, on a dense cluster: the record's rows are sorted across
+    the pieces, and the fixed-point spread scales by what each piece then holds."""
+    import torch
+
+    from nufft_3d_gb300 import nufft_3d
+    rng = np.random.default_rng(11)
+    om = np.concatenate([rng.normal(0, 0.6, (3, 9000)), rng.uniform(-8, 7, (3, 4000))], axis=1)
+    obj = nufft_3d(om, 16, J=6, density_iters=0, tap_table=1, spread_table=0, samples_per_block=64)
+    assert obj.tap_table_bytes > 0 and obj.spread_table_bytes == 0
+    ref = NufftRef(om, 16, J=6, density_iters=0)
+    y = np.abs(rng.standard_normal((om.shape[1], nc))) + 1j * np.abs(rng.standard_normal((om.shape[1], nc)))
+    a = obj.aNUFT(torch.from_numpy(np.ascontiguousarray(y.T).astype(np.complex64)).cuda()).cpu().numpy()
+    r = ref.aNUFT(y)
+    a = a.transpose(3, 2, 1, 0)
+    assert np.linalg.norm(a - r.reshape(a.shape)) < 1e-5 * np.linalg.norm(r)
