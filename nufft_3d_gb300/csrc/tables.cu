@@ -620,7 +620,7 @@ k_spread_rows(const float2 *__restrict__ ks, float2 *__restrict__ G, int nc, int
         };
         // A step's lines are summed by themselves: a quarter of the additions to
         // the long sums, whose rounding grows with their number (64^3 koosh
-        // ball, 8 coils: error against FP64 1.29e-7 -> 1.23e-7, the time as before).
+        // ball, 8 coils: error against FP64 1.65e-7 -> 1.32e-7, the time as before).
         float2 sum4[NQ][NU * NV];
         auto line = [&](const float4 w, unsigned sx, bool first) {
             auto mad = [&](float2 x, float2 y, float2 c) { return first ? __fmul2_rn(x, y) : __ffma2_rn(x, y, c); };
@@ -754,10 +754,11 @@ int configure_spread_tab_kernels()
 // Pieces of at most cap samples: runs of slabs of one column, or shares of a
 // larger slab; most samples first (the heavy centre of radial k-space starts
 // early).  ext: slabs of each piece.  A larger slab is dealt to pieces of up to
-// kSpreadCap whatever cap is: every one of them adds to the same few points of
-// the grid, and the rounding of those sums grows with their number (64^3 koosh
-// ball, 8 coils, shares of 431 samples: error against FP64 2.2e-7, of 1664
-// 1.3e-7; one coil 124 and 129 us).
+// twice cap: every one of them adds to the same few points of the grid, and the
+// rounding of those sums grows with their number, while a larger share holds
+// up the block that takes it (64^3 koosh ball, 262144 samples, cap 431; error
+// against FP64 of 8 coils and adjoint of one coil: shares of 431 1.9e-7, 124 us,
+// of 862 1.3e-7, 123 us, of 1664 1.2e-7, 129 us).
 static void make_spread_pieces(const nufft3d_plan *p, int cap, std::vector<int4> &pcs, std::vector<int> &ext)
 {
     const Geom &g = p->geom;
@@ -780,7 +781,7 @@ static void make_spread_pieces(const nufft3d_plan *p, int cap, std::vector<int4>
         if (c == 0) continue;
         if (start >= 0 && (i / col_slabs != start / col_slabs || i - start >= max_slabs || count + c > cap)) close(last + 1);
         if (c > cap) {
-            const int nb = (c + kSpreadCap - 1) / kSpreadCap;
+            const int share = std::min(kSpreadCap, 2 * cap), nb = (c + share - 1) / share;
             for (int b = 0; b < nb; ++b)
                 runs.push_back({make_int4((int)(off + b), (c - b + nb - 1) / nb | nb << kCountBits, 0, i), 1});
         } else {
@@ -815,7 +816,7 @@ int build_spread_table(nufft3d_plan *p, int mode, cudaStream_t s)
     if (mode == 0 || p->gw == nullptr || p->nnz == 0) return NUFFT3D_SUCCESS;
     const Geom &g = p->geom;
     // Runs for about four pieces a multiprocessor where the samples are few (64^3
-    // x 1 coil, 262144 samples: 85 us, with the largest pieces 99 us).  A 2-D piece holds
+    // x 1 coil, 262144 samples: 80 us, with the largest pieces 99 us).  A 2-D piece holds
     // a whole tile of 38 x 38 points however few its samples are, so there
     // smaller pieces only add points (256^2 x 8 coils: 27 us, four a
     // multiprocessor 41 us).
