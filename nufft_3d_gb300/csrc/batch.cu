@@ -679,13 +679,16 @@ extern "C" int nufft3d_batch_destroy(nufft3d_batch *b)
     clear_error();
     if (!b) return NUFFT3D_SUCCESS;
     {
+        // (the plans may be gone already: a host program tears its objects down in
+        // any order, and the device's work covers theirs)
         NUFFT_DEVICE_LOCK;
-        cudaStreamSynchronize(b->own);
-        for (int v = 0; v < b->nvol; ++v)
-            if (b->plans[v]->own_stream) cudaStreamSynchronize(b->plans[v]->own_stream);
+        int prev = -1;
+        cudaGetDevice(&prev);
+        if (prev != b->device) cudaSetDevice(b->device);
         cudaDeviceSynchronize();
+        free_batch(b);
+        if (prev >= 0 && prev != b->device) cudaSetDevice(prev);
     }
-    free_batch(b);
     delete b;
     return NUFFT3D_SUCCESS;
 }

@@ -68,3 +68,15 @@ def test_batch_rejects_mixed_kernels(cuda):
     c = nufft_3d(om, 16, "J", 6, "u", 1.5)   # same ceil(J/2), different alpha
     with pytest.raises(Exception, match="kernel"):
         NufftBatch([a.share(), c], [1, 1])
+
+
+def test_objects_closed_before_their_batch(cuda):
+    """Objects closed before their batch, as at the end of a program: the batch frees what is its own."""
+    om = synth.koosh_ball(16, 16, 200)
+    objs = [nufft_3d(om, 16, "J", 6, density_iters=0) for _ in range(2)]
+    batch = NufftBatch(objs, [1, 2])
+    ks = batch.forward([cuda.randn(c, 16, 16, 16, dtype=cuda.complex64, device="cuda") for c in (1, 2)])
+    for o in objs:
+        o.close()
+    batch.close()
+    assert all(bool(cuda.isfinite(cuda.view_as_real(k)).all()) for k in ks)
