@@ -256,8 +256,10 @@ int nufft3d_inverse_x0_host(nufft3d_plan *plan, const float *raw_host, float *x_
  * gives.  plans[v] must be distinct handles (nufft3d_plan_share for repeated
  * trajectories) sharing the kernel (J, u, alpha, radial) and 2-D/3-D; the batch
  * uses their work buffers, so do not use those handles concurrently with it.
- * The batch reads the stored H (tap_table) and the stored H' (spread_table)
- * when every volume has it, and otherwise evaluates the kernel for all. */
+ * A volume's passes read the stored H (tap_table) and the stored H'
+ * (spread_table) that its plan holds, in launches of its own; passes without,
+ * and those of volumes too small to gain from it, share one launch per coil
+ * width that evaluates the kernel. */
 typedef struct nufft3d_batch nufft3d_batch;
 int nufft3d_batch_create(nufft3d_plan *const *plans, const int *nc, int nvol, nufft3d_batch **batch);
 int nufft3d_batch_destroy(nufft3d_batch *batch);

@@ -1,13 +1,13 @@
 """Batched operators over many volumes (different N, trajectories, coils).
 
 `NufftBatch([obj_1, ..., obj_n], [nc_1, ..., nc_n])` runs fNUFT, aNUFT and the
-CG iNUFT of every volume with one kernel launch per stage (libnufft3d's
+CG iNUFT of every volume with few kernel launches per stage (libnufft3d's
 nufft3d_batch_*).  Each volume's result equals its own object's.  Objects
 must be distinct plan handles (use ``obj.share()`` to repeat a trajectory)
 with the same J, kernel type and 2-D/3-D.  Tensors are torch CUDA tensors in
 the layouts of ``nufft_3d`` (images (nc, N3, N2, N1), samples (nc, M)).
-The batch reads the stored H and the stored H' when every volume has it, and
-otherwise evaluates the kernel for all.
+A volume's passes read the stored tables that its plan holds; passes without
+share one launch that evaluates the kernel.
 """
 from __future__ import annotations
 

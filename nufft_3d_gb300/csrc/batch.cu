@@ -1,9 +1,10 @@
 // Batched operators over many volumes of different sizes and coil counts.
 //
-// Each stage of fNUFT / aNUFT / iprojection is one launch for the whole batch:
-// the launch's blocks come from a table of (volume, block, coil offset)
+// Stages of fNUFT / aNUFT / iprojection are launches for the whole batch: a
+// launch's blocks come from a table of (volume, block, coil offset)
 // entries and each block reads its volume's descriptor (geometry, tables,
-// buffers) from device memory.  Volumes use the work buffers of their own plan
+// buffers) from device memory.  The line passes of larger volumes and the
+// interpolation from a volume's stored tables are launches of their own.  Volumes use the work buffers of their own plan
 // handle, so a batch needs one handle per volume (nufft3d_plan_share gives
 // several handles on one trajectory).  All volumes must share the kernel
 // half-width R = ceil(J/2), the kernel type (radial or separable) and 2-D/3-D.
@@ -32,6 +33,11 @@ struct BatchSys {
     int first, nblk;  // this system's blocks in the vector-kernel table
 };
 
+constexpr int kSideStreams = 8;  // most streams of the volumes' own interpolation launches
+// Ranges of records taken as one by the 2-D gathers: a range loads its tile's
+// plane anew, which a single volume pays for more blocks at work (32 volumes of
+// 160^2, 100000 radial / random samples, 8 coils: 917 / 1005 us in single ranges).
+constexpr int kMerge2d = 4;
 constexpr int kVecChunk = 8192;  // elements per vector-kernel block
 constexpr int kS = 8;            // per-system scalars
 enum { B_RR, B_BN2, B_ALPHA, B_BETA, B_DONE, B_ITERS, B_TOL };
@@ -43,7 +49,6 @@ using namespace nufft3d;
 struct nufft3d_batch {
     int device = 0, nvol = 0, R = 0, radial = 1, is2d = 0, cb = 8;
     bool rare = false;
-    bool stored_h = false, stored_ht = false;  // every volume's plan holds its stored H, its stored H'
     std::vector<nufft3d_plan *> plans;
     std::vector<int> nc;
     // descriptor arrays (device) and their host mirrors
@@ -65,14 +70,31 @@ struct nufft3d_batch {
     CUtensorMap *d_tmaps = nullptr;     // their device copy (start of the descriptor buffer)
     int *work = nullptr;                // work counter of the persistent interpolation launches
     std::vector<BatchInterp> h_gat, h_spr;
-    // interpolation launch groups: one per coil-pass width
+    // interpolation passes by direction (0 spread, 1 gather): those that read a
+    // stored table, by volume, most work first, and launch groups of the others,
+    // one per coil-pass width
+    struct Pass {
+        int c0, cb;
+    };
+    struct Stored {
+        int v;
+        bool aside;  // on a side stream
+        int64_t weight;
+        std::vector<Pass> passes;
+    };
+    std::vector<Stored> stored[2];
     struct IGroup {
         int cb;
         int4 *tab;
         int n;
         size_t smem;
     };
-    std::vector<IGroup> igroups;
+    std::vector<IGroup> igroups[2];
+    std::vector<char> shared_gather;    // the volume has a gather pass in a launch group
+    // streams that the volumes' own launches run on, beside the batch's
+    std::vector<cudaStream_t> side;
+    std::vector<cudaEvent_t> side_done;
+    cudaEvent_t fork = nullptr;
     BatchPerm *pout = nullptr, *pin = nullptr;
     std::vector<BatchPerm> h_pout, h_pin;
     int4 *ptab = nullptr;
@@ -270,6 +292,22 @@ static void fill_fft(nufft3d_batch *b, int v, BatchFFT *d, int stage)
     }
 }
 
+// Whether a gather pass that can read the volume's stored H is a launch of its
+// own, or shares the launch that evaluates the weights: where a launch holds a
+// few microseconds of work, sharing it gains more than the table.  Batches of 32
+// volumes, forward of radial / random samples in us, own and shared: 16^3 (64
+// tiles), 8192 samples, one coil 318 / 294, 239 / 263, 4 coils 332 / 385, 332 /
+// 360, 8 coils 408 / 488, 470 / 513; 24^3 (216 tiles), 8000 samples, one coil
+// 413 / 473, 465 / 622.  A plane of a 2-D tile is the whole tile, so that short
+// ranges of records load it again and again: 160^2, 100000 samples, one coil 521
+// / 584, 434 / 449, 4 coils 790 / 856, 633 / 656, 8 coils 912 / 1000, 1021 / 1046;
+// 64^2 (16 tiles), 6400, 8 coils 231 / 233, 164 / 167.
+static bool own_gather(const nufft3d_plan *p, int cb)
+{
+    const int64_t tiles = (int64_t)p->geom.nt[0] * p->geom.nt[1] * p->geom.nt[2];
+    return cb >= 8 ? tiles >= 64 : !p->geom.is2d && tiles >= 128;
+}
+
 static int64_t fft_blocks(const nufft3d_plan *p, const BatchFFT &d, int stage, int nc)
 {
     if (stage == FX || stage == IX) return (int64_t)d.N23 * ((nc + kMaxLineCoilsHost - 1) / kMaxLineCoilsHost);
@@ -337,7 +375,7 @@ static void set_io(nufft3d_batch *b, int mode, const float2 *const *in, float2 *
         // grid reallocated between calls never leaves a stale map)
         g.tmap_ok = 0;
         g.tmaps = b->d_tmaps + 4 * v;
-        for (int lw = 1; lw < 4 && !b->stored_h; ++lw)
+        for (int lw = 1; lw < 4 && b->shared_gather[v]; ++lw)
             if (encode_gather_map(p, S.G, b->nc[v], 1 << lw, &b->h_tmaps[4 * v + lw])) g.tmap_ok |= 1 << lw;
         g.scale = mode == 2 ? (float)(1.0 / (double)p->nnz) : (float)(1.0 / std::sqrt((double)p->nnz));
         g.wsample = mode == 2 ? p->d : nullptr;
@@ -418,27 +456,50 @@ static int run_fft_chains(nufft3d_batch *b, bool forward, cudaStream_t s)
     return NUFFT3D_SUCCESS;
 }
 
+static int run_stored(nufft3d_batch *b, bool gather, const nufft3d_batch::Stored &st, cudaStream_t s)
+{
+    const BatchInterp &g = gather ? b->h_gat[st.v] : b->h_spr[st.v];
+    for (auto &q : st.passes)
+        NUFFT_TRY(gather ? launch_gather_tab(b->plans[st.v], g.in, g.out, g.nc, q.c0, q.cb, g.scale, g.wsample,
+                                             b->is2d ? kMerge2d : 1, s)
+                         : launch_spread_tab(b->plans[st.v], g.in, g.out, g.nc, q.c0, q.cb, s));
+    return NUFFT3D_SUCCESS;
+}
+
+// Passes that read a volume's stored table are launches of their own: side by
+// side on a few streams where that gains, since a small volume's launch fills a
+// few multiprocessors and lasts as long as its longest chain of records or
+// pieces.  Gathers always gain (32 volumes of 16^3, 8 coils, forward 1804 -> 659
+// us; 4 of 64^3 and 96^3, 4 to 11 coils 2663 -> 2570), spreads that have fewer
+// pieces than there are multiprocessors (64 volumes of 16^3, 8 coils, adjoint
+// 1678 -> 920 us), while larger ones beside each other lose (three of 96^3, 96^3
+// and 64^3, 6, 7 and 5 coils 2425 -> 3979 us).  The other passes share one launch
+// per coil width.
 static int run_interp(nufft3d_batch *b, bool gather, cudaStream_t s)
 {
-    if (gather && b->stored_h) {
-        // each volume's own persistent launch over its stored H
-        for (int v = 0; v < b->nvol; ++v) {
-            const BatchInterp &g = b->h_gat[v];
-            NUFFT_TRY(launch_gather(b->plans[v], g.in, g.out, g.nc, g.scale, g.wsample, s));
-        }
-        return NUFFT3D_SUCCESS;
-    }
-    if (!gather && b->stored_ht) {
-        for (int v = 0; v < b->nvol; ++v) {
-            const BatchInterp &g = b->h_spr[v];
-            NUFFT_TRY(launch_spread(b->plans[v], g.in, g.out, g.nc, s));
-        }
-        return NUFFT3D_SUCCESS;
-    }
-    for (auto &g : b->igroups)
-        NUFFT_TRY(launch_interp_batch(gather, g.cb, b->R, b->radial, gather ? b->gat : b->spr, g.tab, g.n, g.smem,
-                                      b->plans[0]->kb, b->work, b->plans[0]->sm_count, s));
-    return NUFFT3D_SUCCESS;
+    const auto &own = b->stored[gather];
+    const auto &groups = b->igroups[gather];
+    size_t aside = 0;
+    for (auto &o : own) aside += o.aside;
+    const size_t ns = own.size() + !groups.empty() < 2 ? 0 : std::min(aside, b->side.size());
+    if (ns) NUFFT_CUDA_TRY(cudaEventRecord(b->fork, s));
+    int st = NUFFT3D_SUCCESS;
+    for (size_t i = 0; i < ns && st == NUFFT3D_SUCCESS; ++i)
+        if (cudaStreamWaitEvent(b->side[i], b->fork, 0) != cudaSuccess)
+            st = fail(NUFFT3D_ERR_CUDA, "batch: side stream");
+    size_t turn = 0;
+    for (auto &o : own)
+        if (st == NUFFT3D_SUCCESS) st = run_stored(b, gather, o, ns && o.aside ? b->side[turn++ % ns] : s);
+    for (auto &g : groups)
+        if (st == NUFFT3D_SUCCESS)
+            st = launch_interp_batch(gather, g.cb, b->R, b->radial, gather ? b->gat : b->spr, g.tab, g.n, g.smem,
+                                     b->plans[0]->kb, b->work, b->plans[0]->sm_count, s);
+    // joined also after a failure: a capture must not end with open branches
+    for (size_t i = 0; i < ns; ++i)
+        if (cudaEventRecord(b->side_done[i], b->side[i]) != cudaSuccess ||
+            cudaStreamWaitEvent(s, b->side_done[i], 0) != cudaSuccess)
+            if (st == NUFFT3D_SUCCESS) st = fail(NUFFT3D_ERR_CUDA, "batch: side stream");
+    return st;
 }
 
 static int run_fwd_chain(nufft3d_batch *b, cudaStream_t s)
@@ -467,6 +528,9 @@ static void free_batch(nufft3d_batch *b)
     b->frees.clear();
     if (b->stage) cudaFreeHost(b->stage);
     if (b->up_done) cudaEventDestroy(b->up_done);
+    if (b->fork) cudaEventDestroy(b->fork);
+    for (cudaEvent_t e : b->side_done) cudaEventDestroy(e);
+    for (cudaStream_t q : b->side) cudaStreamDestroy(q);
     if (b->own) cudaStreamDestroy(b->own);
 }
 
@@ -566,26 +630,42 @@ extern "C" int nufft3d_batch_create(nufft3d_plan *const *plans, const int *nc, i
         b->chain[v] = (int64_t)b->h_fft[FX][v].N23 * nch >= 4 * (int64_t)plans[v]->sm_count;
     }
     {
-        // interpolation: (volume, piece, first coil), heaviest pieces first
+        // interpolation: passes that read a stored table, by volume, and
+        // (volume, piece, first coil) entries of the others, heaviest pieces first
         struct E {
             int count;
             int4 e;
         };
-        std::vector<E> ents;
+        std::vector<E> ents[2];
         int maxcand = 0;
         b->h_gat.resize(nvol);
         b->h_spr.resize(nvol);
+        b->shared_gather.assign(nvol, 0);
         for (int v = 0; v < nvol; ++v) {
             nufft3d_plan *p = plans[v];
             std::vector<int4> blk(p->n_blocks);
             if (p->n_blocks && cudaMemcpy(blk.data(), p->blocks, sizeof(int4) * p->n_blocks, cudaMemcpyDeviceToHost) != cudaSuccess)
                 return bail(fail(NUFFT3D_ERR_CUDA, "batch: reading tile pieces failed"));
-            for (int64_t k = 0; k < p->n_blocks; ++k)
-                for (int c0 = 0; c0 < nc[v]; c0 += cb) {
-                    int w = 1;  // this chunk's width: smallest power of two covering its coils
-                    while (w < nc[v] - c0 && w < cb) w *= 2;
-                    ents.push_back({blk[k].z, make_int4(v, (int)k, c0, w)});
+            nufft3d_batch::Stored own[2];
+            for (int c0 = 0; c0 < nc[v]; c0 += cb) {
+                int w = 1;  // this pass's width: smallest power of two covering its coils
+                while (w < nc[v] - c0 && w < cb) w *= 2;
+                for (int gather = 0; gather < 2; ++gather) {
+                    if (gather ? gather_reads_table(p) && own_gather(p, w) : spread_reads_table(p, w)) {
+                        own[gather].passes.push_back({c0, w});
+                        continue;
+                    }
+                    if (gather) b->shared_gather[v] = 1;
+                    for (int64_t k = 0; k < p->n_blocks; ++k) ents[gather].push_back({blk[k].z, make_int4(v, (int)k, c0, w)});
                 }
+            }
+            for (int gather = 0; gather < 2; ++gather) {
+                if (own[gather].passes.empty()) continue;
+                own[gather].v = v;
+                own[gather].aside = gather || p->n_spread_pieces < p->sm_count;
+                own[gather].weight = p->nnz * nc[v];
+                b->stored[gather].push_back(own[gather]);
+            }
             BatchInterp d;
             std::memset(&d, 0, sizeof(d));
             d.samples = p->samples;
@@ -594,34 +674,54 @@ extern "C" int nufft3d_batch_create(nufft3d_plan *const *plans, const int *nc, i
             d.kb = p->kb;
             d.cand = p->cand_desc;
             d.status = plan_status(p);  // timeouts are reported on the volume's plan
-            if (v == 0) b->stored_h = b->stored_ht = true;
-            if (p->nnz > 0 && !p->gw) b->stored_h = false;
-            if (p->nnz > 0 && !p->spread_ent) b->stored_ht = false;
             d.nc = nc[v];
             b->h_gat[v] = d;
             b->h_spr[v] = d;
             maxcand = std::max(maxcand, p->n_cand);
         }
-        std::stable_sort(ents.begin(), ents.end(), [](const E &a, const E &c) { return a.count > c.count; });
-        for (int w = cb; w >= 1; w /= 2) {
-            std::vector<int4> tab;
-            for (auto &e : ents)
-                if (e.e.w == w) tab.push_back(make_int4(e.e.x, e.e.y, e.e.z, 0));
-            if (tab.empty()) continue;
-            nufft3d_batch::IGroup ig;
-            ig.cb = w;
-            ig.n = (int)tab.size();
-            const size_t plane = smem_plane_bytes(b->R, w);
-            const size_t iplane = (size_t)(((plane / (w * sizeof(float2)) + 29) / 32) * 32 + 2) * w * 2 * sizeof(int);
-            // + tile alignment; the spread keeps its candidates as packed pairs
-            ig.smem = std::max(plane, iplane) +
-                      std::max(cand_smem_bytes(maxcand), cand_pairs_bytes(b->h_spr[0].cand)) + 128;
-            int s2 = dalloc(b, &ig.tab, tab.size());
-            if (s2 != NUFFT3D_SUCCESS) return bail(s2);
-            if (cudaMemcpy(ig.tab, tab.data(), tab.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess)
-                return bail(fail(NUFFT3D_ERR_CUDA, "batch table upload failed"));
-            b->igroups.push_back(ig);
+        size_t most = 0;
+        for (int gather = 0; gather < 2; ++gather) {
+            auto &own = b->stored[gather];
+            std::stable_sort(own.begin(), own.end(), [](const nufft3d_batch::Stored &x, const nufft3d_batch::Stored &y) {
+                return x.weight > y.weight;
+            });
+            size_t n = 0;
+            for (auto &o : own) n += o.aside;
+            most = std::max(most, n);
+            auto &es = ents[gather];
+            std::stable_sort(es.begin(), es.end(), [](const E &x, const E &y) { return x.count > y.count; });
+            for (int w = cb; w >= 1; w /= 2) {
+                std::vector<int4> tab;
+                for (auto &e : es)
+                    if (e.e.w == w) tab.push_back(make_int4(e.e.x, e.e.y, e.e.z, 0));
+                if (tab.empty()) continue;
+                nufft3d_batch::IGroup ig;
+                ig.cb = w;
+                ig.n = (int)tab.size();
+                const size_t plane = smem_plane_bytes(b->R, w);
+                const size_t iplane = (size_t)(((plane / (w * sizeof(float2)) + 29) / 32) * 32 + 2) * w * 2 * sizeof(int);
+                // + tile alignment; the spread keeps its candidates as packed pairs
+                ig.smem = std::max(plane, iplane) +
+                          std::max(cand_smem_bytes(maxcand), cand_pairs_bytes(b->h_spr[0].cand)) + 128;
+                int s2 = dalloc(b, &ig.tab, tab.size());
+                if (s2 != NUFFT3D_SUCCESS) return bail(s2);
+                if (cudaMemcpy(ig.tab, tab.data(), tab.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess)
+                    return bail(fail(NUFFT3D_ERR_CUDA, "batch table upload failed"));
+                b->igroups[gather].push_back(ig);
+            }
         }
+        for (size_t i = 0; i < std::min<size_t>(most, kSideStreams); ++i) {
+            cudaStream_t q = nullptr;
+            if (cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking) != cudaSuccess)
+                return bail(fail(NUFFT3D_ERR_CUDA, "batch stream"));
+            b->side.push_back(q);
+            cudaEvent_t e = nullptr;
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+                return bail(fail(NUFFT3D_ERR_CUDA, "batch event"));
+            b->side_done.push_back(e);
+        }
+        if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
+            return bail(fail(NUFFT3D_ERR_CUDA, "batch event"));
     }
     {
         std::vector<int4> tab;

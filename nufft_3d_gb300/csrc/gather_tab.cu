@@ -111,6 +111,7 @@ struct GatherArgs {
     const GatherRec *recs;
     const int2 *chunks;  // record ranges
     int nchunks;
+    int merge;           // ranges taken as one
     const uint32_t *grow;
     const float4 *gw;    // [chunk][8]: weights of entries l (x, y) and l + 8 (z, w)
     const uint32_t *gi;  // [chunk][8]: their points, l in the low half
@@ -361,7 +362,11 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
             const int b = lane == 0 ? atomicAdd(a.work, 1) : 0;
             return __shfl_sync(0xffffffffu, b, 0);
         };
-        auto range = [&](int b) { return b < a.nchunks ? __ldg(&a.chunks[b]) : make_int2(0, 0); };
+        auto range = [&](int b) {
+            const int lo = b * a.merge;
+            if (lo >= a.nchunks) return make_int2(0, 0);
+            return make_int2(__ldg(&a.chunks[lo]).x, __ldg(&a.chunks[min(lo + a.merge, a.nchunks) - 1]).y);
+        };
         // Records are read 32 at a time, one a lane, a batch ahead: a global load
         // takes longer than a record does.
         int2 cur = make_int2(0, 0);       // the rest of the range that the batches come from
@@ -1044,14 +1049,14 @@ static int launch_rows(nufft3d_plan *p, GatherArgs &a, const CUtensorMap &m, cud
     a.rbytes = (unsigned)smem;
     smem += (size_t)a.PS * sizeof(uint32_t);  // plane offsets
     if (a.S < a.npl) return fail(NUFFT3D_ERR_UNSUPPORTED, "stored H: plane ring too small");
-    const int grid = std::min(a.nchunks, interp_grid_sms(p) * GatherCfg<CB>::MINB);
+    const int grid = std::min((a.nchunks + a.merge - 1) / a.merge, interp_grid_sms(p) * GatherCfg<CB>::MINB);
     k_gather_rows<CB, NPW><<<grid, GatherCfg<CB>::WARPS * 32, smem, s>>>(a, m);
     NUFFT_CUDA_TRY(cudaGetLastError());
     return NUFFT3D_SUCCESS;
 }
 
 int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int c0, int cb, float scale,
-                      const float *ws, cudaStream_t s)
+                      const float *ws, int merge, cudaStream_t s)
 {
     const Geom &g = p->geom;
     GatherArgs a;
@@ -1067,6 +1072,7 @@ int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int 
     a.recs = p->grecs;
     a.chunks = p->gchunks;
     a.nchunks = p->n_gchunks;
+    a.merge = merge;
     a.grow = p->grow;
     a.gw = p->gw;
     a.gi = p->gi;

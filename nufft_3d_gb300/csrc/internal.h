@@ -408,11 +408,15 @@ int launch_weight_sum(nufft3d_plan *p, cudaStream_t s);
 // the stored tables serve this plan (8-coil passes, R <= 3)
 bool tap_table_applies(const nufft3d_plan *p);
 // stored H (gather_tab.cu): plan-time build, and the gather of coils
-// c0..c0+cb-1 that reads it (cb 1, 2, 4 or 8)
+// c0..c0+cb-1 that reads it (cb 1, 2, 4 or 8; all coils of an odd count below
+// 8 in one pass), taking `merge` ranges of its records at a time
 int build_gather_table(nufft3d_plan *p, int mode, cudaStream_t s);
 int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int c0, int cb, float scale,
-                      const float *ws, cudaStream_t s);
+                      const float *ws, int merge, cudaStream_t s);
 int configure_gather_tab_kernels();
+// whether a pass (of cb coils) reads the plan's stored H (H')
+bool gather_reads_table(const nufft3d_plan *p);
+bool spread_reads_table(const nufft3d_plan *p, int cb);
 // the map of the grid for bulk copies of one plane of a padded tile, cb coils
 bool encode_plane_map(const nufft3d_plan *p, const float2 *G, int nc, int cb, CUtensorMap *m);
 // spread: G += H' ks (G zeroed by caller)

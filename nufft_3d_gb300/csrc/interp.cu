@@ -1242,6 +1242,17 @@ static int dispatch(nufft3d_plan *p, const float2 *in, float2 *out, int nc, int 
 
 constexpr int64_t kSpreadTabSamples = 32768;
 
+bool gather_reads_table(const nufft3d_plan *p) { return p->gw != nullptr; }
+
+// The stored H', where its FP32 sums, whose last bits depend on the order in
+// which pieces meet in the grid, buy time: plans of fewer samples and coils keep
+// the fixed-point spread, whose sums at those sizes are exact and equal bit for
+// bit from call to call.
+bool spread_reads_table(const nufft3d_plan *p, int cb)
+{
+    return p->spread_ent != nullptr && (cb >= 8 || p->nnz >= kSpreadTabSamples);
+}
+
 template <bool GATHER>
 static int interp(nufft3d_plan *p, const float2 *in, float2 *out, int nc, float scale,
                   const float *ws, cudaStream_t s)
@@ -1253,16 +1264,12 @@ static int interp(nufft3d_plan *p, const float2 *in, float2 *out, int nc, float 
         int cb = 1;
         while (cb < rem && cb < cmax) cb *= 2;
         int st;
-        if (GATHER && p->gw) {  // the stored H, any coil width
-            NUFFT_TRY(launch_gather_tab(p, in, out, nc, c0, cb, scale, ws, s));
+        if (GATHER && gather_reads_table(p)) {
+            NUFFT_TRY(launch_gather_tab(p, in, out, nc, c0, cb, scale, ws, 1, s));
             if (cb > rem) break;
             continue;
         }
-        // The stored H', where its FP32 sums, whose last bits depend on the order
-        // in which pieces meet in the grid, buy time: plans of fewer samples and
-        // coils keep the fixed-point spread, whose sums at those sizes are exact
-        // and equal bit for bit from call to call.
-        if (!GATHER && p->spread_ent && (cb >= 8 || p->nnz >= kSpreadTabSamples)) {
+        if (!GATHER && spread_reads_table(p, cb)) {
             NUFFT_TRY(launch_spread_tab(p, in, out, nc, c0, cb, s));
             if (cb > rem) break;
             continue;

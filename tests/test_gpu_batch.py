@@ -80,3 +80,43 @@ def test_objects_closed_before_their_batch(cuda):
         o.close()
     batch.close()
     assert all(bool(cuda.isfinite(cuda.view_as_real(k)).all()) for k in ks)
+
+
+@pytest.mark.parametrize("shape,nvol,ncs", [
+    ((16, 16, 16), 9, (1, 2, 8)),      # small volumes: narrow passes share a launch, 8-coil ones are their own
+    ((24, 20, 30), 11, (1, 3, 12)),    # more volumes than side streams, a pass of each kind in one volume
+    ((40, 36, 1), 10, (1, 8)),         # 2-D: few tiles, all shared
+    ((140, 128, 1), 3, (2, 8, 9)),     # 2-D: 8-coil passes of their own, ranges of records merged
+])
+def test_many_volumes(cuda, shape, nvol, ncs):
+    """Volumes with both tables, with the stored H alone and with none, in one batch on a stream of its own: each
+    equals its own object."""
+    torch = cuda
+    rng = np.random.default_rng(nvol)
+    tables = [dict(tap_table=1, spread_table=1), dict(tap_table=1, spread_table=0), dict(tap_table=0)]
+    objs, xs, ys = [], [], []
+    for v in range(nvol):
+        m = 1500 + 977 * v
+        om = np.stack([rng.uniform(-n / 2, n / 2 - 1, m) if n > 1 else np.zeros(m) for n in shape])
+        if v % 2:  # a dense centre
+            om = om * rng.random(m) ** 2
+        objs.append(nufft_3d(om, shape, "J", 6, density_iters=3, **(tables[v % 3] if v > 4 else tables[0])))
+        nc = ncs[v % len(ncs)]
+        xs.append(torch.randn(nc, *shape[::-1], dtype=torch.complex64, device="cuda"))
+        ys.append(torch.randn(nc, m, dtype=torch.complex64, device="cuda"))
+    single_k = [o.fNUFT(x) for o, x in zip(objs, xs)]
+    single_a = [o.aNUFT(y) for o, y in zip(objs, ys)]
+    single_i = [o.iNUFT(y, 4, 0.05, solver="cg", tol=0.0) for o, y in zip(objs, ys)]
+    batch = NufftBatch(objs, [x.shape[0] for x in xs])
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        for _ in range(2):
+            ks, xa, xi = batch.forward(xs), batch.adjoint(ys), batch.inverse(ys, 4, 0.05, tol=0.0)
+    stream.synchronize()
+    for v in range(nvol):
+        assert rel(ks[v], single_k[v]) < TOL_OP, v
+        assert rel(xa[v], single_a[v]) < TOL_OP, v
+        assert rel(xi[v], single_i[v]) < TOL_IMG, v
+        objs[v].check_status(stream)
+    batch.close()
