@@ -53,6 +53,14 @@ __device__ __forceinline__ void tma_load_3d(unsigned dst, const CUtensorMap *map
                  : "memory");
 }
 
+// bytes (a multiple of 16) from 16-byte aligned src to 16-byte aligned dst
+__device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
 // Bounded wait for the phase of the given parity (at most `polls` polls);
 // false if it expired.
 constexpr int kDrainPolls = 1 << 22;

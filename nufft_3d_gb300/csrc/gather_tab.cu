@@ -177,9 +177,31 @@ __device__ __forceinline__ size_t grid_plane(const GatherArgs &a, int z)
     return (size_t)(a.small ? ring_wrap(z, a.K[2]) : near_wrap(z, a.K[2])) * a.K[1] * a.K[0];
 }
 
-// Planes [z0, z0 + n) of the padded tile, into ring slots slot, slot + 1, ...,
-// where bulk copies do not apply: tiles that wrap around the grid edge by
-// 16-byte asynchronous copies of coil pairs ...
+// Planes [z0, z0 + n) of a padded tile at (ox, oy) that wraps around the grid
+// edge, into ring slots slot, slot + 1, ...  Where the pass takes every coil, a
+// row of points is one contiguous run, or two: bulk copies that the lanes of one
+// warp issue.  (Runs start at even points and have an even number, whole 16-byte
+// units: K1 and P0 are even and so is ox, see tile_shift.)
+template <int CB>
+__device__ __forceinline__ void load_rows(const GatherArgs &a, unsigned ring, unsigned pbytes, int slot, int ox, int oy,
+                                          int z0, int n, int lane, unsigned bar)
+{
+    constexpr unsigned SLOT = CB * 8;
+    if (lane == 0) mbar_expect_bytes(bar, (unsigned)n * (unsigned)(a.P0 * a.P1) * SLOT);
+    __syncwarp();
+    const int x0 = near_wrap(ox, a.K[0]), n0 = min(a.P0, a.K[0] - x0);
+    for (int q = lane; q < n * a.P1; q += 32) {
+        const int t = q / a.P1, y = q - t * a.P1;
+        const int sl = slot + t < a.S ? slot + t : slot + t - a.S;
+        const float2 *row = a.G + (grid_plane(a, z0 + t) + (size_t)near_wrap(oy + y, a.K[1]) * a.K[0]) * CB;
+        const unsigned dst = ring + (unsigned)sl * pbytes + (unsigned)(y * a.P0) * SLOT;
+        bulk_load(dst, row + (size_t)x0 * CB, (unsigned)n0 * SLOT, bar);
+        if (n0 < a.P0) bulk_load(dst + (unsigned)n0 * SLOT, row, (unsigned)(a.P0 - n0) * SLOT, bar);
+    }
+}
+
+// The others are copied by the producer warps: 16-byte asynchronous copies of
+// coil pairs ...
 template <int CB>
 __device__ __forceinline__ void copy_pairs(const GatherArgs &a, const uint32_t *poff, unsigned ring, unsigned pbytes,
                                            int slot, int z0, int n, int t, int nt)
@@ -239,7 +261,9 @@ __device__ __forceinline__ void copy_coils(const GatherArgs &a, const uint32_t *
     }
 }
 
-template <int CB, int NPW>
+// ROWS: a pass of every coil, see load_rows; else NPW producer warps copy the
+// tiles that wrap.
+template <int CB, int NPW, bool ROWS>
 __global__ void __launch_bounds__(GatherCfg<CB>::WARPS * 32, GatherCfg<CB>::MINB)
 k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUtensorMap tmap)
 {
@@ -464,6 +488,8 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
                         }
                     }
                     copied = false;
+                } else if constexpr (ROWS) {
+                    load_rows<CB>(a, ring, pbytes, slot, rec.ox, rec.oy, z0, rec.nload, lane, fb);
                 } else {
                     copied = true;
                     async = pairs;
@@ -549,12 +575,13 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
         auto next_task = [&]() -> bool {
             int t = -2;  // expired, -1: no more tasks
             if (lane == 0) {
+                const int mine = task;
+                task = atomicAdd(&ctl[1], 1);
                 for (int i = 0; i < kDrainPolls && t == -2; ++i) {
-                    if (ld_acquire(&ctl[0]) > task) t = task;
-                    else if (ld_acquire(&ctl[2]) <= task || *ab) t = -1;
+                    if (ld_acquire(&ctl[0]) > mine) t = mine;
+                    else if (ld_acquire(&ctl[2]) <= mine || *ab) t = -1;
                     else __nanosleep(50);
                 }
-                task = atomicAdd(&ctl[1], 1);
             }
             t = __shfl_sync(0xffffffffu, t, 0);
             if (t < 0) {
@@ -911,7 +938,7 @@ static void make_records(const nufft3d_plan *p, std::vector<GatherRec> &recs, ui
 
 // Record ranges: each about a sixth of what is left for each multiprocessor
 // (rows, a loaded plane of 14 x 14 points counting as four, or 16 where the
-// tile wraps around the grid edge and is copied piecemeal), so that the last ones are short,
+// tile wraps around the grid edge and takes longer), so that the last ones are short,
 // and at least 128 rows, below which the planes that a range loads anew
 // outweigh its rows.
 static std::vector<int2> make_chunks(const std::vector<GatherRec> &recs, const Geom &g, int sms)
@@ -1041,7 +1068,7 @@ static int ring_planes(const Geom &g, size_t *bytes)
     return S;
 }
 
-template <int CB, int NPW>
+template <int CB, int NPW, bool ROWS>
 static int launch_rows(nufft3d_plan *p, GatherArgs &a, const CUtensorMap &m, cudaStream_t s)
 {
     size_t smem = 0;
@@ -1050,7 +1077,7 @@ static int launch_rows(nufft3d_plan *p, GatherArgs &a, const CUtensorMap &m, cud
     smem += (size_t)a.PS * sizeof(uint32_t);  // plane offsets
     if (a.S < a.npl) return fail(NUFFT3D_ERR_UNSUPPORTED, "stored H: plane ring too small");
     const int grid = std::min((a.nchunks + a.merge - 1) / a.merge, interp_grid_sms(p) * GatherCfg<CB>::MINB);
-    k_gather_rows<CB, NPW><<<grid, GatherCfg<CB>::WARPS * 32, smem, s>>>(a, m);
+    k_gather_rows<CB, NPW, ROWS><<<grid, GatherCfg<CB>::WARPS * 32, smem, s>>>(a, m);
     NUFFT_CUDA_TRY(cudaGetLastError());
     return NUFFT3D_SUCCESS;
 }
@@ -1091,55 +1118,75 @@ int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int 
     const bool odd = nc == a.cb && nc % 2 == 1 && nc < 8;
     if (odd) cb = nc;
     a.use_tma = p->use_tma && encode_plane_map(p, G, nc, cb, &m) ? 1 : 0;
-    // Tiles that wrap around the grid edge are copied by the producer warps, not
-    // by bulk copies.  Four of them instead of one where such tiles are common
-    // (percentage of inner tiles below the limit) gain on the copies what the
-    // consumers lose in warps, the more the wider the pass: forward of 8 coils
-    // at 32^3 (56 % inner, 16384 random samples) 98 -> 76 us, 7 coils at
-    // 88 x 112 x 100 (79 %, 1000003) 2177 -> 1509 us, 5 coils at 128^3 (87 %)
-    // 1922 -> 1734 us; past the limits one is better: 4 coils at 128^3 1568 ->
-    // 1401 us, one coil at 64^3 (76 %, 262144) 155 -> 111 us.  A 2-D plane is a
-    // whole tile of 38 x 38 points (324 x 98, 3 coils: 166 -> 58 us, with the
-    // shorter ranges of make_chunks).
+    // Tiles that wrap around the grid edge are loaded row by row where a pass takes
+    // every coil (gather of random samples in us, against copies by one and by
+    // four producer warps: 8 coils at 96^3, 1000000 samples, 718, 824, 741, 65536 at
+    // 64^3, J = 4, 212, 244, 228; 5 coils on 88 x 112 x 100 415, 657, 569; one coil at
+    // 64^3, 262144, 100, 122, 148; radial samples, one coil at 48^3 51, 67, 61; a
+    // bulk copy for each point of the other passes took 2 to 5 times as long as
+    // the copies).
+    if (p->use_tma && nc == cb && !a.small) {
+        switch (cb) {
+        case 1: return launch_rows<1, 1, true>(p, a, m, s);
+        case 2: return launch_rows<2, 1, true>(p, a, m, s);
+        case 3: return launch_rows<3, 1, true>(p, a, m, s);
+        case 4: return launch_rows<4, 1, true>(p, a, m, s);
+        case 5: return launch_rows<5, 1, true>(p, a, m, s);
+        case 7: return launch_rows<7, 1, true>(p, a, m, s);
+        default: return launch_rows<8, 1, true>(p, a, m, s);
+        }
+    }
+    // Otherwise the producer warps copy them: four of them instead of one where
+    // such tiles are common (percentage of inner tiles below the limit) gain on
+    // the copies what the consumers lose in warps, the more the wider the pass.
+    // One against four, radial / random samples, 8 coils: at 64^3 (76 % inner)
+    // 174 / 315, 160 / 247 us, at 80^3 (81 %) 284 / 524, 292 / 459, at 96^3 (84 %)
+    // 458 / 824, 501 / 741; 4 coils at 48^3 (69 %) 84 / 129, 79 / 113, at 64^3 144 / 225,
+    // 150 / 230.  A 2-D plane is a whole tile of 38 x 38 points.  (An odd number of
+    // coils takes this path without bulk copies, or on a grid of a tile or two.)
     const int inner = 100 * std::max(0, g.nt[0] - 2) * std::max(0, g.nt[1] - 2) / (g.nt[0] * g.nt[1]);
-    const bool copies = !a.use_tma || g.is2d || inner < (cb <= 2 ? 50 : cb % 2 == 0 ? 79 : cb == 3 ? 85 : 90);
+    const bool copies = !a.use_tma || g.is2d || inner < (cb == 2 ? 50 : 79);
     switch (cb) {
-    case 1: return copies ? launch_rows<1, 4>(p, a, m, s) : launch_rows<1, 1>(p, a, m, s);
-    case 2: return copies ? launch_rows<2, 4>(p, a, m, s) : launch_rows<2, 1>(p, a, m, s);
-    case 3: return copies ? launch_rows<3, 4>(p, a, m, s) : launch_rows<3, 1>(p, a, m, s);
-    case 5: return copies ? launch_rows<5, 4>(p, a, m, s) : launch_rows<5, 1>(p, a, m, s);
-    case 7: return copies ? launch_rows<7, 4>(p, a, m, s) : launch_rows<7, 1>(p, a, m, s);
-    case 4: return copies ? launch_rows<4, 4>(p, a, m, s) : launch_rows<4, 1>(p, a, m, s);
-    default: return copies ? launch_rows<8, 4>(p, a, m, s) : launch_rows<8, 1>(p, a, m, s);
+    case 1: return launch_rows<1, 4, false>(p, a, m, s);
+    case 2: return copies ? launch_rows<2, 4, false>(p, a, m, s) : launch_rows<2, 1, false>(p, a, m, s);
+    case 3: return launch_rows<3, 4, false>(p, a, m, s);
+    case 4: return copies ? launch_rows<4, 4, false>(p, a, m, s) : launch_rows<4, 1, false>(p, a, m, s);
+    case 5: return launch_rows<5, 4, false>(p, a, m, s);
+    case 7: return launch_rows<7, 4, false>(p, a, m, s);
+    default: return copies ? launch_rows<8, 4, false>(p, a, m, s) : launch_rows<8, 1, false>(p, a, m, s);
     }
 }
 
-template <int CB, int NPW>
+template <int CB, int NPW, bool ROWS>
 static int allow_rows()
 {
+    auto *k = k_gather_rows<CB, NPW, ROWS>;
     cudaFuncAttributes fa;
-    NUFFT_CUDA_TRY(cudaFuncGetAttributes(&fa, k_gather_rows<CB, NPW>));
-    NUFFT_CUDA_TRY(cudaFuncSetAttribute(k_gather_rows<CB, NPW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    NUFFT_CUDA_TRY(cudaFuncGetAttributes(&fa, k));
+    NUFFT_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         227 * 1024 / GatherCfg<CB>::MINB - 1024 - (int)fa.sharedSizeBytes));
     return NUFFT3D_SUCCESS;
 }
 
 int configure_gather_tab_kernels()
 {
-    NUFFT_TRY((allow_rows<1, 1>()));
-    NUFFT_TRY((allow_rows<1, 4>()));
-    NUFFT_TRY((allow_rows<2, 1>()));
-    NUFFT_TRY((allow_rows<2, 4>()));
-    NUFFT_TRY((allow_rows<3, 1>()));
-    NUFFT_TRY((allow_rows<3, 4>()));
-    NUFFT_TRY((allow_rows<5, 1>()));
-    NUFFT_TRY((allow_rows<5, 4>()));
-    NUFFT_TRY((allow_rows<7, 1>()));
-    NUFFT_TRY((allow_rows<7, 4>()));
-    NUFFT_TRY((allow_rows<4, 1>()));
-    NUFFT_TRY((allow_rows<4, 4>()));
-    NUFFT_TRY((allow_rows<8, 1>()));
-    NUFFT_TRY((allow_rows<8, 4>()));
+    NUFFT_TRY((allow_rows<1, 1, true>()));
+    NUFFT_TRY((allow_rows<2, 1, true>()));
+    NUFFT_TRY((allow_rows<3, 1, true>()));
+    NUFFT_TRY((allow_rows<4, 1, true>()));
+    NUFFT_TRY((allow_rows<5, 1, true>()));
+    NUFFT_TRY((allow_rows<7, 1, true>()));
+    NUFFT_TRY((allow_rows<8, 1, true>()));
+    NUFFT_TRY((allow_rows<1, 4, false>()));
+    NUFFT_TRY((allow_rows<2, 1, false>()));
+    NUFFT_TRY((allow_rows<2, 4, false>()));
+    NUFFT_TRY((allow_rows<3, 4, false>()));
+    NUFFT_TRY((allow_rows<4, 1, false>()));
+    NUFFT_TRY((allow_rows<4, 4, false>()));
+    NUFFT_TRY((allow_rows<5, 4, false>()));
+    NUFFT_TRY((allow_rows<7, 4, false>()));
+    NUFFT_TRY((allow_rows<8, 1, false>()));
+    NUFFT_TRY((allow_rows<8, 4, false>()));
     return NUFFT3D_SUCCESS;
 }
 

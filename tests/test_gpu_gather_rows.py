@@ -101,3 +101,22 @@ def test_rows_move_samples_between_small_pieces(nc):
     r = ref.aNUFT(y)
     a = a.transpose(3, 2, 1, 0)
     assert np.linalg.norm(a - r.reshape(a.shape)) < 1e-5 * np.linalg.norm(r)
+
+
+@pytest.mark.parametrize("nc", [1, 2, 3, 4, 5, 6, 7, 8, 9, 16])
+@pytest.mark.parametrize("N,opts", [
+    ((14, 18, 22), dict(J=6, u=2)),               # one to three tiles an axis, every column at the edge
+    ((12, 26, 10), dict(J=5, u=1.5, radial=0)),   # tiles cut short by the grid
+    ((36, 20, 12), dict(J=2, u=2)),               # odd tile origins moved by one
+    ((50, 44, 1), dict(J=4, u=2)),
+])
+def test_tiles_that_wrap(N, opts, nc):
+    """Samples in the outermost cells of both ends of every axis: rows that wrap in x, in y and in both."""
+    rng = np.random.default_rng(nc)
+    n = np.asarray(N)
+    m = 3000
+    om = np.stack([np.where(rng.random(m) < 0.5, -v / 2 + rng.random(m), v / 2 - 1 - rng.random(m)) if v > 1
+                   else np.zeros(m) for v in n])
+    om[:, ::3] = np.stack([rng.uniform(-v / 2, v / 2 - 1, om[:, ::3].shape[1]) if v > 1
+                           else np.zeros(om[:, ::3].shape[1]) for v in n])
+    _case(N, om, nc, opts)
