@@ -297,9 +297,10 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
     __syncthreads();
     const unsigned pbytes = (unsigned)a.PS * SLOT;
     // A wait that runs out is reported and ends the block's work.  A warp takes
-    // that decision as one (lane 0 waits and tells the others, or they vote): a
-    // lane that left alone would leave the others at the next warp-wide
-    // instruction.
+    // that decision as one, by vote: a lane that left alone would leave the
+    // others at the next warp-wide instruction.  (Lane 0 alone at the polls, the
+    // others waiting for what it tells them, took longer: 2 to 15 % of a small
+    // volume's gather.)
     volatile int *const ab = &ctl[3];
     auto give_up = [&]() {
         if (lane == 0) {
@@ -349,6 +350,7 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
                     if (lane == 0) st_release(&ctl[0], tend[st]);
                     ++landed;
                     copy = BoundedWait();
+                    continue;
                 } else {
                     ++copy.failed;
                 }
@@ -449,15 +451,14 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
             rows += rec.nrows;
             while (d < rr && (rr - d >= kStages || send[d % kStages] - a.npl < endp + rec.nload - a.S ||
                               rows - srow[d % kStages] > kRowsAhead)) {
-                int ok = 0;
-                if (lane == 0) {
-                    const int want = stask[d % kStages];
-                    for (int t = 0; t < kDrainPolls && !ok && !*ab; ++t) {
-                        ok = ld_acquire(&finished[d % kStages]) - want >= 0;
-                        if (!ok) __nanosleep(50);
-                    }
+                const int want = stask[d % kStages];
+                bool ok = false;
+                for (int t = 0; t < kDrainPolls; ++t) {
+                    ok = __all_sync(0xffffffffu, ld_acquire(&finished[d % kStages]) - want >= 0) != 0;
+                    if (ok || ended()) break;
+                    __nanosleep(50);
                 }
-                if (!__shfl_sync(0xffffffffu, ok, 0)) {
+                if (!ok) {
                     give_up();
                     live = false;
                     break;
@@ -465,7 +466,6 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
                 ++d;
             }
             if (!live) break;
-            __syncwarp();  // what lane 0 saw finished is finished for every lane
             const int st = rr % kStages;
             const unsigned fb = full + 8 * st;
             const bool pairs = kPaired<CB> && a.pairs;
@@ -573,22 +573,20 @@ k_gather_rows(const __grid_constant__ GatherArgs a, const __grid_constant__ CUte
         int task = lane == 0 ? atomicAdd(&ctl[1], 1) : 0;
         // Starts the loads of the warp's next task; false at the end.
         auto next_task = [&]() -> bool {
-            int t = -2;  // expired, -1: no more tasks
-            if (lane == 0) {
-                const int mine = task;
-                task = atomicAdd(&ctl[1], 1);
-                for (int i = 0; i < kDrainPolls && t == -2; ++i) {
-                    if (ld_acquire(&ctl[0]) > mine) t = mine;
-                    else if (ld_acquire(&ctl[2]) <= mine || *ab) t = -1;
-                    else __nanosleep(50);
-                }
+            const int t = __shfl_sync(0xffffffffu, task, 0);
+            if (lane == 0) task = atomicAdd(&ctl[1], 1);
+            bool ok = false, end = false;
+            for (int i = 0; i < kDrainPolls; ++i) {
+                ok = __all_sync(0xffffffffu, ld_acquire(&ctl[0]) > t) != 0;
+                if (ok) break;
+                end = __any_sync(0xffffffffu, ld_acquire(&ctl[2]) <= t || *ab != 0) != 0;
+                if (end) break;
+                __nanosleep(50);
             }
-            t = __shfl_sync(0xffffffffu, t, 0);
-            if (t < 0) {
-                if (t == -2) give_up();
+            if (!ok) {
+                if (!end) give_up();  // expired
                 return false;
             }
-            __syncwarp();  // what lane 0 saw published is seen by every lane
             const GatherTask &f = tasks[t % kTasks];
             const int4 g = *reinterpret_cast<const int4 *>(&f);
             stage = g.w;
@@ -1145,7 +1143,7 @@ int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int 
     // 150 / 230.  A 2-D plane is a whole tile of 38 x 38 points.  (An odd number of
     // coils takes this path without bulk copies, or on a grid of a tile or two.)
     const int inner = 100 * std::max(0, g.nt[0] - 2) * std::max(0, g.nt[1] - 2) / (g.nt[0] * g.nt[1]);
-    const bool copies = !a.use_tma || g.is2d || inner < (cb == 2 ? 50 : 79);
+    const bool copies = !a.use_tma || g.is2d || inner < (cb == 8 ? 79 : cb == 4 ? 72 : 50);
     switch (cb) {
     case 1: return launch_rows<1, 4, false>(p, a, m, s);
     case 2: return copies ? launch_rows<2, 4, false>(p, a, m, s) : launch_rows<2, 1, false>(p, a, m, s);
