@@ -68,7 +68,8 @@ typedef struct nufft3d_opts {
                           tile order, read by the gather passes of fNUFT
                           (see spread_table for H'): 1 = build it, 0 = evaluate
                           the kernel on the fly, -1 = auto (default: build it
-                          when it takes at most half of the free device memory) */
+                          when it takes at most half of the free device memory;
+                          2-D plans of few samples evaluate all the same) */
     int wait_polls;    /* polls of each bounded wait of the interpolation
                           kernels (the tile copy of the gather) before it gives
                           up and reports NUFFT3D_ERR_TIMEOUT (default 2^22, well

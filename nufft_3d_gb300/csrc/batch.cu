@@ -651,7 +651,7 @@ extern "C" int nufft3d_batch_create(nufft3d_plan *const *plans, const int *nc, i
                 int w = 1;  // this pass's width: smallest power of two covering its coils
                 while (w < nc[v] - c0 && w < cb) w *= 2;
                 for (int gather = 0; gather < 2; ++gather) {
-                    if (gather ? gather_reads_table(p) && own_gather(p, w) : spread_reads_table(p, w)) {
+                    if (gather ? p->gw && own_gather(p, w) : spread_reads_table(p, w)) {
                         own[gather].passes.push_back({c0, w});
                         continue;
                     }

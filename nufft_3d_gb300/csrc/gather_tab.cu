@@ -1122,8 +1122,12 @@ int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int 
     // 64^3, J = 4, 212, 244, 228; 5 coils on 88 x 112 x 100 415, 657, 569; one coil at
     // 64^3, 262144, 100, 122, 148; radial samples, one coil at 48^3 51, 67, 61; a
     // bulk copy for each point of the other passes took 2 to 5 times as long as
-    // the copies).
-    if (p->use_tma && nc == cb && !a.small) {
+    // the copies).  Eight coils on a grid of mostly outer tiles are left to the four
+    // warps below: with a record of few rows the copies of all eight land sooner
+    // (26^3, 49 % inner, radial / random 29 / 45 us row by row, 25 / 41; 48^3, 69 %, 62 /
+    // 124, 66 / 119).
+    const int inner = 100 * std::max(0, g.nt[0] - 2) * std::max(0, g.nt[1] - 2) / (g.nt[0] * g.nt[1]);
+    if (p->use_tma && nc == cb && !a.small && (cb != 8 || g.is2d || inner >= 60)) {
         switch (cb) {
         case 1: return launch_rows<1, 1, true>(p, a, m, s);
         case 2: return launch_rows<2, 1, true>(p, a, m, s);
@@ -1142,7 +1146,6 @@ int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int 
     // 458 / 824, 501 / 741; 4 coils at 48^3 (69 %) 84 / 129, 79 / 113, at 64^3 144 / 225,
     // 150 / 230.  A 2-D plane is a whole tile of 38 x 38 points.  (An odd number of
     // coils takes this path without bulk copies, or on a grid of a tile or two.)
-    const int inner = 100 * std::max(0, g.nt[0] - 2) * std::max(0, g.nt[1] - 2) / (g.nt[0] * g.nt[1]);
     const bool copies = !a.use_tma || g.is2d || inner < (cb == 8 ? 79 : cb == 4 ? 72 : 50);
     switch (cb) {
     case 1: return launch_rows<1, 4, false>(p, a, m, s);

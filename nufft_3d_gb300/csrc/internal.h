@@ -350,6 +350,7 @@ struct nufft3d_plan {
     float4 *gw = nullptr;
     uint32_t *gi = nullptr;
     int64_t tap_bytes = 0;
+    bool tap_always = false;     // asked for: read by every gather
     // stored H' (tables.cu): pieces (first sample, count and stride, first
     // step, first slab), the warps' first steps and segments, the lines'
     // weights and slots, the segments' grid points and steps
@@ -415,7 +416,7 @@ int launch_gather_tab(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, int 
                       const float *ws, int merge, cudaStream_t s);
 int configure_gather_tab_kernels();
 // whether a pass (of cb coils) reads the plan's stored H (H')
-bool gather_reads_table(const nufft3d_plan *p);
+bool gather_reads_table(const nufft3d_plan *p, int cb);
 bool spread_reads_table(const nufft3d_plan *p, int cb);
 // the map of the grid for bulk copies of one plane of a padded tile, cb coils
 bool encode_plane_map(const nufft3d_plan *p, const float2 *G, int nc, int cb, CUtensorMap *m);

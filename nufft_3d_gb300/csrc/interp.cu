@@ -1242,7 +1242,20 @@ static int dispatch(nufft3d_plan *p, const float2 *in, float2 *out, int nc, int 
 
 constexpr int64_t kSpreadTabSamples = 32768;
 
-bool gather_reads_table(const nufft3d_plan *p) { return p->gw != nullptr; }
+// The stored H, but for 2-D plans of the automatic mode whose samples no
+// multiprocessor has many of (its largest piece, or its share of all): a tile's
+// plane is the whole tile, and staging it for the evaluating kernel's larger
+// blocks costs less.  Gather in us, table and evaluated, one coil / 3 / 8: 324 x 98,
+// 10000 random samples (100 a multiprocessor) 17 / 17 / 19, 12 / 14 / 16; 200 x 160,
+// 40000 (307 in the largest piece) 18 / 19 / 19, 15 / 18 / 22; 150000 (1154) 22 / 27 /
+// 34, 26 / 32 / 38; radial samples, 160^2, 32000 (1500) 19 / 20 / 19, 36 / 46 / 62.
+bool gather_reads_table(const nufft3d_plan *p, int cb)
+{
+    if (!p->gw) return false;
+    if (!p->geom.is2d || p->tap_always) return true;
+    const int64_t load = std::max<int64_t>(p->piece_samples, p->nnz / p->sm_count);
+    return load > (cb >= 8 ? 256 : 400);
+}
 
 // The stored H', where its FP32 sums, whose last bits depend on the order in
 // which pieces meet in the grid, buy time: plans of fewer samples and coils keep
@@ -1264,7 +1277,7 @@ static int interp(nufft3d_plan *p, const float2 *in, float2 *out, int nc, float 
         int cb = 1;
         while (cb < rem && cb < cmax) cb *= 2;
         int st;
-        if (GATHER && gather_reads_table(p)) {
+        if (GATHER && gather_reads_table(p, cb)) {
             NUFFT_TRY(launch_gather_tab(p, in, out, nc, c0, cb, scale, ws, 1, s));
             if (cb > rem) break;
             continue;

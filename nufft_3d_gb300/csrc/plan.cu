@@ -922,6 +922,7 @@ extern "C" int nufft3d_plan_create(const double *om, int64_t M, const int32_t *N
         return fail(NUFFT3D_ERR_CUDA, "cudaStreamCreate failed");
     }
     p->wait_polls = o.wait_polls;
+    p->tap_always = o.tap_table == 1;
     int st = dmalloc(&p->work, 16, nullptr);  // per handle: handles may run concurrently
     if (st == NUFFT3D_SUCCESS && cudaMemset(p->work, 0, 16 * sizeof(int)) != cudaSuccess)
         st = fail(NUFFT3D_ERR_CUDA, "cannot clear the plan's work buffer");
@@ -1012,6 +1013,7 @@ extern "C" int nufft3d_plan_share(const nufft3d_plan *src, nufft3d_plan **out)
         return fail(NUFFT3D_ERR_CUDA, "cudaStreamCreate failed");
     }
     p->wait_polls = src->wait_polls;
+    p->tap_always = src->tap_always;
     if (dmalloc(&p->work, 16, nullptr) != NUFFT3D_SUCCESS || cudaMemset(p->work, 0, 16 * sizeof(int)) != cudaSuccess) {
         std::string msg = p->work ? std::string("cannot clear the handle's work buffer") : nufft3d_last_error();
         if (p->work) cudaFree(p->work);

@@ -120,3 +120,19 @@ def test_table_shared_handle_and_solver(cuda):
         assert rel(im, imr) < TOL_IMG
     finally:
         h.close()
+
+
+@pytest.mark.parametrize("shape,m", [((40, 60, 1), 3000), ((200, 120, 1), 40000), ((64, 64, 1), 60000)])
+@pytest.mark.parametrize("nc", [1, 2, 5, 8])
+def test_2d_plans_read_the_table_by_their_load(shape, m, nc):
+    """The automatic mode evaluates where few samples fall to a multiprocessor and reads the stored H elsewhere; asked
+    for, it is always read.  All agree to the order of the additions."""
+    import torch
+
+    from nufft_3d_gb300 import nufft_3d
+    rng = np.random.default_rng(nc)
+    om = np.stack([rng.uniform(-n / 2, n / 2 - 1, m) if n > 1 else np.zeros(m) for n in shape])
+    x = torch.randn(nc, *shape[::-1], dtype=torch.complex64, device="cuda")
+    k = [nufft_3d(om, shape, J=6, density_iters=0, tap_table=t).fNUFT(x) for t in (-1, 0, 1)]
+    for a in k[1:]:
+        assert float((a - k[0]).abs().norm() / k[0].abs().norm()) < 1e-6
