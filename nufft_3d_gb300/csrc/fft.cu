@@ -1063,15 +1063,27 @@ int launch_fft_batch_p(const BatchFFTParams &P, int kind, size_t smem, bool rare
 // have 16-wide line chunks, else 0.
 int batch_four_step(int K, bool all_vec16) { return all_vec16 ? four_step_r1(K, 16) : 0; }
 
+// The x pass in two register phases takes 16 (row, coil) lines a block: too few
+// of them leave the chip to a few blocks of long register DFTs, and the Stockham
+// form's block a row is faster.  Forward x pass in us, two phases / Stockham: K =
+// 500, 250 rows, one coil 15 / 9, 3 coils 14 / 11, 8 coils 13 / 17; K = 200, 100
+// rows, one coil 12 / 9, 8 coils 10 / 10; K = 840, 300 rows, 3 coils 17 / 14; short
+// lines gain at once (K = 56, 784 rows, one coil 8 / 12).
+static TwoStep two_step_x(const FFTDesc &fd, int64_t nlines, int nv)
+{
+    if (fd.n > 128 && nlines < 768 && line_smem(nv, fd.n) <= 64 * 1024) return TwoStep();
+    return two_step(fd.n);
+}
+
 int launch_fx(nufft3d_plan *p, const float2 *img, float2 *B1, int nc, cudaStream_t s)
 {
     const int N1 = p->N[0], N23 = p->N[1] * p->N[2];
     const FFTDesc &fd = p->fft[0];
     if (const int r1 = four_step_r1(fd.n, 16))
         return launch_xline4<false>(r1, img, B1, p->U, fd, N1, N23, nc, 1.f, nullptr, 0.f, s);
-    const TwoStep t = two_step(fd.n);
-    if (t.r1) return launch_xline2<false>(t, img, B1, p->U, fd, N1, N23, nc, 1.f, nullptr, 0.f, s);
     const int nv = nc < kMaxLineCoils ? nc : kMaxLineCoils;
+    const TwoStep t = two_step_x(fd, (int64_t)N23 * nc, nv);
+    if (t.r1) return launch_xline2<false>(t, img, B1, p->U, fd, N1, N23, nc, 1.f, nullptr, 0.f, s);
     dim3 grid(N23, (nc + kMaxLineCoils - 1) / kMaxLineCoils);
     if (needs_rare(fd))
         k_fx<true><<<grid, kFftThreads, line_smem(nv, fd.n), s>>>(img, p->U, B1, N1, N23, nc, fd);
@@ -1088,9 +1100,9 @@ int launch_ix(nufft3d_plan *p, const float2 *B1, float2 *img, int nc, float scal
     const FFTDesc &fd = p->fft[0];
     if (const int r1 = four_step_r1(fd.n, 16))
         return launch_xline4<true>(r1, B1, img, p->U, fd, N1, N23, nc, scale, addend, add_coef, s);
-    const TwoStep t = two_step(fd.n);
-    if (t.r1) return launch_xline2<true>(t, B1, img, p->U, fd, N1, N23, nc, scale, addend, add_coef, s);
     const int nv = nc < kMaxLineCoils ? nc : kMaxLineCoils;
+    const TwoStep t = two_step_x(fd, (int64_t)N23 * nc, nv);
+    if (t.r1) return launch_xline2<true>(t, B1, img, p->U, fd, N1, N23, nc, scale, addend, add_coef, s);
     dim3 grid(N23, (nc + kMaxLineCoils - 1) / kMaxLineCoils);
     if (needs_rare(fd))
         k_ix<true><<<grid, kFftThreads, line_smem(nv, fd.n), s>>>(B1, p->U, img, N1, N23, nc, fd, scale,

@@ -78,3 +78,27 @@ def test_long_lengths_without_a_split(N, u, nc):
     a = a.transpose(3, 2, 1, 0)
     assert np.linalg.norm(f - fr.reshape(f.shape)) < 1e-5 * np.linalg.norm(fr)
     assert np.linalg.norm(a - ar.reshape(a.shape)) < 1e-5 * np.linalg.norm(ar)
+
+
+@pytest.mark.parametrize("K", [132, 150, 168, 182, 196, 200, 210, 242, 308, 338, 420, 484, 512, 572, 700, 896, 1024])
+def test_x_lengths_with_many_lines(K):
+    """x passes of at least 768 lines take the two register phases at every length; with fewer the block-a-row form."""
+    import torch
+
+    from nufft_3d_gb300 import nufft_3d
+    rng = np.random.default_rng(K)
+    n = 2 * -(-K // 4)
+    u = K / n - 1e-9
+    for N, nc in (((n, 16, 16), 3), ((n, 14, 10), 5)):  # 768 and 700 lines
+        om = np.stack([rng.uniform(-v / 2, v / 2 - 1, 1200) for v in N])
+        obj = nufft_3d(om, N, J=4, u=u, density_iters=0)
+        ref = NufftRef(om, N, J=4, u=u, density_iters=0)
+        assert ref.K[0] == K
+        x = rng.standard_normal((*N, nc)) + 1j * rng.standard_normal((*N, nc))
+        y = rng.standard_normal((1200, nc)) + 1j * rng.standard_normal((1200, nc))
+        f = obj.fNUFT(torch.from_numpy(x.transpose(3, 2, 1, 0).astype(np.complex64)).cuda()).cpu().numpy()
+        a = obj.aNUFT(torch.from_numpy(np.ascontiguousarray(y.T).astype(np.complex64)).cuda()).cpu().numpy()
+        fr, ar = ref.fNUFT(x), ref.aNUFT(y)
+        assert np.linalg.norm(f.T - fr.reshape(f.T.shape)) < 1e-5 * np.linalg.norm(fr)
+        a = a.transpose(3, 2, 1, 0)
+        assert np.linalg.norm(a - ar.reshape(a.shape)) < 1e-5 * np.linalg.norm(ar)
