@@ -147,14 +147,15 @@ def ncu_figures():
         return json.load(f)
 
 
-def ncu_traffic(kernel):
-    """DRAM bytes per launch of `kernel` at this workload from the committed ncu summary."""
-    return ncu_figures().get(kernel)
+# the kernels of the interpolation stages; figures of any other are not theirs
+STAGE_KERNELS = {"gather": "k_gather_rows", "spread": "k_spread_rows"}
 
 
-def ncu_sm_side(kernel):
-    """Issue and shared-memory utilisation of `kernel` from the committed ncu summary."""
-    return ncu_figures().get("sm_side", {}).get(kernel)
+def ncu_figure(stage, key):
+    """A figure of the committed ncu summary (traffic: DRAM bytes per launch at this workload; sm_side: issue and
+    data-path utilisation), or None where the summary is of another kernel than the one that runs."""
+    f = ncu_figures().get(stage)
+    return f.get(key) if isinstance(f, dict) and f.get("kernel") == STAGE_KERNELS.get(stage) else None
 
 
 def dist_init(backend="nccl"):
@@ -239,14 +240,41 @@ def uneven_volumes(n_vol=48, seed=3):
     return vols
 
 
+def batch_work_bytes(N, M, nc):
+    """Bytes of a volume's buffers in a batched solve at K = 2N: grid and line-pass intermediates, sorted samples,
+    eight solver vectors, the raw data and two images."""
+    return 8 * nc * ((8 + 4 + 2) * N ** 3 + M + 8 * N ** 3 + M + 2 * N ** 3)
+
+
+def table_options(M, room):
+    """The stored H and H' (1.7 KB a sample at J = 6) where they take less than `room` bytes, else neither."""
+    return {} if 1700 * M < room else {"tap_table": 0, "spread_table": 0}
+
+
+def extra(leg, *args):
+    """Result of an extra leg; one that fails is reported in its place and does not take the others with it."""
+    import torch
+    try:
+        return leg(*args)
+    except Exception as e:
+        return {"error": "%s: %s" % (type(e).__name__, str(e)[:300])}
+    finally:
+        torch.cuda.empty_cache()
+
+
 def bench_batched(maxit=20, damp=1e-3):
-    """48 uneven volumes reconstructed by the batched CG (one launch per
-    stage for all volumes) against the same volumes one after another."""
+    """48 uneven volumes reconstructed by the batched CG against the same
+    volumes one after another.  All are resident at once: a volume gets its
+    stored tables while the work buffers of all of them still fit beside."""
     import torch
     from nufft_3d_gb300 import NufftBatch, nufft_3d
     vols = uneven_volumes()
-    objs = [nufft_3d(om, N, "J", 6, density_iters=20) for om, N, _, _ in vols]
     ncs = [nc for _, _, nc, _ in vols]
+    work = sum(batch_work_bytes(N, om.size // 3, nc) for om, N, nc, _ in vols)
+    objs = []
+    for om, N, _, _ in vols:
+        room = torch.cuda.mem_get_info()[0] - work - (12 << 30)
+        objs.append(nufft_3d(om, N, "J", 6, density_iters=20, **table_options(om.size // 3, room)))
     g = torch.Generator(device="cuda").manual_seed(0)
     raws = [torch.randn((nc, o.M), dtype=torch.complex64, device="cuda", generator=g) for o, nc in zip(objs, ncs)]
     batch = NufftBatch(objs, ncs)
@@ -272,6 +300,7 @@ def bench_batched(maxit=20, damp=1e-3):
             "coil_samples": samples, "batched_volumes_per_s": round(len(vols) / t_b, 3),
             "sequential_volumes_per_s": round(len(vols) / t_s, 3), "speedup": round(t_s / t_b, 3),
             "batched_s": round(t_b, 3), "sequential_s": round(t_s, 3),
+            "volumes_with_tables": sum(o.tap_table_bytes > 0 for o in objs),
             "max_rel_l2_batched_vs_single": err}
 
 
@@ -613,18 +642,18 @@ def main():
     d = stages[dom]
     roof = {"bound": "hbm", "kernel": dom, "achieved": d["achieved_gbs"], "peak": hbm, "unit": "GB/s",
             "frac": round(d["achieved_gbs"] / hbm, 4), "peak_source": src,
-            "traffic": ncu_traffic(dom), "algo_bytes_per_launch": d["algo_bytes_per_launch"],
-            "sm_side": ncu_sm_side(dom)}
-    if "gather" in stages and obj.tap_table_bytes and nc >= 8:
-        # the stored H read by the 8-coil gather passes, beside its algorithmic bytes
-        hb = obj.tap_table_bytes * (nc // 8)
+            "traffic": ncu_figure(dom, "traffic"), "algo_bytes_per_launch": d["algo_bytes_per_launch"],
+            "sm_side": ncu_figure(dom, "sm_side")}
+    if "gather" in stages and obj.tap_table_bytes:
+        # the stored H read by every gather pass, beside its algorithmic bytes
+        hb = obj.tap_table_bytes * -(-nc // 8)
         g = stages["gather"]
         g["stored_h_bytes"] = hb
         g["achieved_gbs_with_stored_h"] = round((g["algo_bytes_per_launch"] + hb) /
                                                 (g["ms_per_step"] / 1e3 / max(1, g["launches"] // args.steps)) / 1e9, 1)
-    if "spread" in stages and obj.spread_table_bytes and nc >= 8:
-        # the stored H' read by the 8-coil spread passes, beside its algorithmic bytes
-        hb = obj.spread_table_bytes * (nc // 8)
+    if "spread" in stages and obj.spread_table_bytes and (nc >= 8 or obj.nnz >= 32768):
+        # the stored H' read by every spread pass, beside its algorithmic bytes
+        hb = obj.spread_table_bytes * -(-nc // 8)
         g = stages["spread"]
         g["stored_h_t_bytes"] = hb
         g["achieved_gbs_with_stored_h_t"] = round((g["algo_bytes_per_launch"] + hb) /
@@ -661,13 +690,13 @@ def main():
             "stages": stages,
             "clocks": clk.summary()}
     if not args.no_extras and ws == 1:
-        line["fft_comparator"] = bench_cufft(args.N, int(obj.K[0]), nc, ours_fft)
+        line["fft_comparator"] = extra(bench_cufft, args.N, int(obj.K[0]), nc, ours_fft)
         obj.close()
         del x, k, x2
         torch.cuda.empty_cache()
-        line["batched"] = bench_batched()
-        line["serving"] = bench_serving()
-        line["large_cg"] = bench_large_cg()
+        line["batched"] = extra(bench_batched)
+        line["serving"] = extra(bench_serving)
+        line["large_cg"] = extra(bench_large_cg)
     if want_acc:
         line["cpu_baseline"], line["accuracy"] = cpu_baseline(om, args.N, im, k_host, a_host)
     print(json.dumps(line))
