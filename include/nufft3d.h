@@ -127,8 +127,9 @@ int nufft3d_plan_destroy(nufft3d_plan *plan);
  * shared d. */
 int nufft3d_plan_share(const nufft3d_plan *src, nufft3d_plan **plan);
 
-/* Caps the persistent interpolation kernels (gather and spread: one block
- * per multiprocessor) of this handle at `sms` multiprocessors; 0 = all.  The
+/* Caps the persistent interpolation kernels (gather and spread) of this handle
+ * at `sms` multiprocessors, with one block for each whatever the coil count
+ * (uncapped, narrow passes run several on each); 0 = all.  The
  * others stay free for kernels on other streams -- e.g. the host-link-bound
  * stages of another handle's host-pointer call, so that two threads calling
  * nufft3d_forward_host / _adjoint_host on two handles overlap one call's

@@ -1074,7 +1074,7 @@ static int launch_rows(nufft3d_plan *p, GatherArgs &a, const CUtensorMap &m, cud
     a.rbytes = (unsigned)smem;
     smem += (size_t)a.PS * sizeof(uint32_t);  // plane offsets
     if (a.S < a.npl) return fail(NUFFT3D_ERR_UNSUPPORTED, "stored H: plane ring too small");
-    const int grid = std::min((a.nchunks + a.merge - 1) / a.merge, interp_grid_sms(p) * GatherCfg<CB>::MINB);
+    const int grid = std::min((a.nchunks + a.merge - 1) / a.merge, interp_grid_blocks(p, GatherCfg<CB>::MINB));
     k_gather_rows<CB, NPW, ROWS><<<grid, GatherCfg<CB>::WARPS * 32, smem, s>>>(a, m);
     NUFFT_CUDA_TRY(cudaGetLastError());
     return NUFFT3D_SUCCESS;

@@ -432,6 +432,9 @@ int launch_spread_tab(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, int 
 int configure_spread_tab_kernels();
 // multiprocessors the persistent interpolation kernels of a handle may use
 int interp_grid_sms(const nufft3d_plan *p);
+// blocks of a persistent kernel of which per_sm fit on a multiprocessor: under a
+// cap one for each that it allows, since more would land on the others
+int interp_grid_blocks(const nufft3d_plan *p, int per_sm);
 // user [M nc] <-> sorted [nnz][nc]
 int launch_permute_out(nufft3d_plan *p, const float2 *ks, float2 *k, int nc, float scale,
                        cudaStream_t s);

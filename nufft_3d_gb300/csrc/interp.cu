@@ -1212,6 +1212,12 @@ int interp_grid_sms(const nufft3d_plan *p)
     return p->interp_sms > 0 && p->interp_sms < p->sm_count ? p->interp_sms : p->sm_count;
 }
 
+int interp_grid_blocks(const nufft3d_plan *p, int per_sm)
+{
+    const int sms = interp_grid_sms(p);
+    return sms < p->sm_count ? sms : sms * per_sm;
+}
+
 bool tap_table_applies(const nufft3d_plan *p) { return p->coils_per_pass == 8 && p->geom.R <= 3; }
 
 template <bool GATHER, int CB, bool RADIAL>

@@ -708,7 +708,7 @@ template <int CB>
 static int launch_rows(nufft3d_plan *p, const float2 *ks, float2 *G, int nc, int c0, cudaStream_t s)
 {
     const size_t smem = spread_smem<CB>(p->spread_cap);
-    const int64_t grid = std::min<int64_t>(p->n_spread_pieces, (int64_t)interp_grid_sms(p) * SpreadCfg<CB>::MINB);
+    const int64_t grid = std::min<int64_t>(p->n_spread_pieces, (int64_t)interp_grid_blocks(p, SpreadCfg<CB>::MINB));
     k_spread_rows<CB><<<(unsigned)grid, kBundleWarps * 32, smem, s>>>(
         ks, G, nc, c0, std::min(CB, nc - c0), p->spread_pieces, (int)p->n_spread_pieces, p->spread_cap,
         p->work + kWorkSpreadTab, p->spread_wstart,

@@ -110,3 +110,36 @@ def test_host_copy_modes_match(cuda):
         assert np.array_equal(k, k0), key          # the gather is deterministic
         assert rel(a, a0) < 1e-6, key              # the grid's float atomics may add in another order
     assert L.nufft3d_plan_set_host_copy(obj.plan, 2) == _lib.ERR_ARG
+
+
+@pytest.mark.parametrize("nc", [1, 2, 3, 4, 5, 8])
+def test_capped_handle_launches_a_block_a_multiprocessor(cuda, nc, tmp_path):
+    """nufft3d_plan_set_sms: the interpolation launches of every coil width have at most that many blocks."""
+    import json
+    torch = cuda
+    N, cap = 64, 40
+    om = synth.koosh_ball(N, 64, 1200)
+    obj = nufft_3d(om, N, "J", 6, density_iters=0, tap_table=1, spread_table=1)
+    x = torch.randn(nc, N, N, N, dtype=torch.complex64, device="cuda")
+    k = obj.fNUFT(x)
+    a = obj.aNUFT(k)
+    _lib.check(_lib.load().nufft3d_plan_set_sms(obj.plan, cap))
+    for _ in range(2):  # (the first trace of a process can come back empty)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            k2 = obj.fNUFT(x)
+            a2 = obj.aNUFT(k)
+            torch.cuda.synchronize()
+    path = str(tmp_path / "trace.json")
+    prof.export_chrome_trace(path)
+    blocks = {}
+    for e in json.load(open(path))["traceEvents"]:
+        grid = e.get("args", {}).get("grid") if e.get("cat") == "kernel" else None
+        if grid:
+            for stage in ("k_gather", "k_spread"):
+                if stage in e["name"]:
+                    blocks[stage] = max(blocks.get(stage, 0), int(np.prod(grid)))
+    if not blocks:
+        pytest.skip("no kernel records from the profiler")
+    assert set(blocks) == {"k_gather", "k_spread"} and all(b <= cap for b in blocks.values()), blocks
+    assert float((k2 - k).abs().norm() / k.abs().norm()) < 1e-6
+    assert float((a2 - a).abs().norm() / a.abs().norm()) < 1e-6
