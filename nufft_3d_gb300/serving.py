@@ -133,13 +133,17 @@ class ReconServer:
         # sorted records, perm, inv, d, d_orig, U, tiles
         b = M * (16 + 4 + 4 + 4 + 4) + N ** 3 * 4 + (K // 8 + 1) ** 3 * 20
         # the stored H and its transpose H' that plans with ceil(J/2) <= 3
-        # build when they fit, sized for sparse trajectories (16384 random
-        # samples, J = 6: 0.83 and 1.17 KB per sample; 8.4 M: 0.73 and 0.87)
+        # build when they fit, bounded from their layouts for any trajectory.
+        # H: 10 bytes a tap, as if no two samples shared a point, rows padded by
+        # half a chunk.  H': 18 bytes for each row of 2 x 2 points that a sample
+        # reaches (about taps / 4 + 0.72 taps^(2/3)), and for the rows themselves,
+        # of which the pieces have up to 0.9 for each grid point with their
+        # halos, 16 bytes of points and up to three entries of padding.
         J = float(req.opts.get("J", 4))
         if int(np.ceil(J / 2)) <= 3:
             taps = 4.0 / 3.0 * np.pi * (J / 2) ** 3 if req.opts.get("radial", 1) else J ** 3
-            b += int(M * ((taps + 4) * 8 + 4))
-            b += int(M * (taps + 24) * 8)
+            b += int(M * (taps + 8) * 10)
+            b += int(M * (taps / 4 + 0.72 * taps ** (2 / 3)) * 18) + int(0.9 * K ** 3 * 70)
         return b
 
     @staticmethod

@@ -135,3 +135,15 @@ def test_low_and_high_gain_requests_merged_match_alone(cuda):
     assert done[0].t_start == done[1].t_start  # one merged solve
     for r, a in zip(done, alone):
         assert rel(r.result, a) < 1e-5, rel(r.result, a)
+
+
+@pytest.mark.parametrize("J", [4, 6])
+@pytest.mark.parametrize("N,m", [(32, 16384), (64, 16384), (128, 16384), (64, 262144), (96, 1500000)])
+def test_table_estimate_covers_any_trajectory(cuda, N, m, J):
+    """Admission counts at least the bytes that the tables take, for sparse random samples (short rows, padded to whole
+    steps) as for dense ones."""
+    rng = np.random.default_rng(N)
+    om = rng.uniform(-N / 2, N / 2 - 1, (3, m))
+    obj = nufft_3d(om, N, "J", J, density_iters=0, tap_table=1, spread_table=1)
+    req = Request(om=om, N=N, raw=None, opts={"J": J})
+    assert obj.tap_table_bytes + obj.spread_table_bytes <= ReconServer._plan_bytes_estimate(req)
