@@ -71,12 +71,13 @@ typedef struct nufft3d_opts {
                           when it takes at most half of the free device memory;
                           2-D plans of few samples evaluate all the same) */
     int wait_polls;    /* polls of each bounded wait of the interpolation
-                          kernels (the tile copy of the gather) before it gives
-                          up and reports NUFFT3D_ERR_TIMEOUT (default 2^22, well
-                          under a second); 0 gives up at once: every bulk tile
-                          copy is then still allowed to land, but its tile is
-                          skipped and the timeout reported, which exercises the
-                          error path without a fault */
+                          kernels (the grid copies of the gather) before it is
+                          reported as NUFFT3D_ERR_TIMEOUT (default 2^22, well
+                          under a second).  The evaluating gather then skips the
+                          tile once its copy has landed; the gather from the
+                          stored H goes on waiting, up to 2^22 polls, and ends
+                          the block's work after that.  0 reports every wait,
+                          which exercises the error path without a fault */
     int spread_table;  /* stored transpose H' (only beside the stored H), read by
                           the spread passes of aNUFT (passes of fewer than 8
                           coils: from 32768 samples on): per piece of at most
@@ -293,8 +294,8 @@ int nufft3d_profile_read(nufft3d_plan *plan, char *buf, int cap);
  * status flag after the work queued on `stream` (the stream the device-pointer
  * calls ran on; NULL = the legacy default stream) and synchronises that
  * stream.  Returns NUFFT3D_ERR_TIMEOUT if a bounded wait in an interpolation
- * kernel expired since the last check (the affected tiles were skipped, so
- * those results are incomplete), else NUFFT3D_SUCCESS.  Device-pointer calls
+ * kernel expired since the last check (tiles may have been skipped: those
+ * results count as incomplete), else NUFFT3D_SUCCESS.  Device-pointer calls
  * (nufft3d_forward, _adjoint, _normal, _inverse*, nufft3d_forward_noalloc and
  * the batch calls, which report on the plans of their volumes) return before
  * their kernels run and report through this call; the host-pointer calls and

@@ -107,11 +107,6 @@ __device__ __forceinline__ int ld_acquire(const int *p)
     return v;
 }
 
-__device__ __forceinline__ void copy_async4(unsigned dst, const void *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-
 __device__ __forceinline__ void copy_async8(unsigned dst, const void *src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");

@@ -29,12 +29,10 @@
 // shares planes with those before it), and asks L2 for the entries ahead.  No
 // barrier spans the block after set-up.
 //
-// Measured at 128^3 x 8 coils: 1.88 ms (one 1024-thread block a tile piece with
-// a barrier on either side, one row a sample: 3.53 ms), of which the waits for
-// planes are a quarter; while they work the consumers move 22 wavefronts a
-// 32-entry step through the L1 data path, which is what bounds them (16 are
-// the points themselves).  One coil at 64^3: 0.08 ms (evaluating the kernel
-// 0.19 ms), 192^3 x 16 coils: 11.0 ms (21.2 ms).
+// Measured at 128^3 x 8 coils: 1.78 ms (one 1024-thread block a tile piece with
+// a barrier on either side, one row a sample: 3.53 ms).  The L1 data path bounds
+// it, 72 % of its peak in a capture at 96^3: 24 shared wavefronts a step of 32
+// entries, 16 of them the points themselves.  192^3 x 16 coils: 11.0 ms (21.2 ms).
 //
 // Table layout: row r holds chunks [grow[r], grow[r+1]) of 16 entries; lane l
 // of the row reads entries l and l + 8 of a chunk as one float4 of gw[8 c + l]
@@ -45,7 +43,7 @@
 //     (l mod NP) ^ k, so the 8 lanes of a row touch all four 16-byte columns
 //     in every load, two lanes each; eight entries hold even points in 0-3 and
 //     odd ones in 4-7 while they can, so the two differ in their half of the
-//     banks (9 % of the wavefronts conflict);
+//     banks (5 % of the wavefronts conflict);
 //   * entries 4-7 store the weights of samples 1, 0, so the first reduction
 //     step (lanes l and l ^ 4) keeps accumulator 0 in every lane;
 //   * the pair rotation makes the next steps keep accumulators by their own
@@ -76,7 +74,7 @@ constexpr int kRowsAhead = 256;  // rows in flight
 
 // Warps, blocks per SM and chunks of a row each lane keeps in flight.  With 8
 // coils the ring takes the whole shared memory, and 16 warps of 128 registers
-// measured faster (1.88 ms at 128^3) than 20 of 96 (2.15 ms) or 24 of 80, which
+// measured faster (1.88 ms at 128^3 then) than 20 of 96 (2.15 ms) or 24 of 80, which
 // spill: the ring leaves the L1 cache too small for spills.  Fewer coils leave
 // room for more blocks, which hide the latency of short records.
 template <int CB>

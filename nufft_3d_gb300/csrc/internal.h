@@ -178,14 +178,14 @@ struct InterpStatus {
     int polls;  // polls of each bounded wait
 };
 
-// A record of the stored-H gather: rows of four samples of one slab of a tile
+// A record of the stored-H gather: rows of two samples of one slab of a tile
 // (origin of the slab's first plane; planes not already in the ring when the
 // record before it was the previous one of the list).
 struct GatherRec {
     int ox, oy, oz, nload;
     uint32_t row0;
     int nrows, s0, ns;
-    uint32_t chunk0, nchunk;  // its entries: chunks of 8
+    uint32_t chunk0, nchunk;  // its entries: chunks of 16
 };
 
 // First cell of tile 0 along x: the padded tile then starts at an even grid
@@ -342,7 +342,7 @@ struct nufft3d_plan {
                                 // plan's status flags (slots kWork*)
     int wait_polls = nufft3d::kDefaultWaitPolls;  // polls of each bounded wait in the gather
     // stored H (gather_tab.cu): records, ranges of records, first chunk of each
-    // row of four samples, weights and points of the entries
+    // row of two samples, weights and points of the entries
     nufft3d::GatherRec *grecs = nullptr;
     int2 *gchunks = nullptr;
     int n_gchunks = 0;
@@ -406,7 +406,7 @@ int launch_gather(nufft3d_plan *p, const float2 *G, float2 *ks, int nc, float sc
                   const float *wsample, cudaStream_t s);
 // plan time: per-block bound on summed weights (blocks[b].w) for the spread
 int launch_weight_sum(nufft3d_plan *p, cudaStream_t s);
-// the stored tables serve this plan (8-coil passes, R <= 3)
+// the stored tables serve this plan (not limited to fewer than 8 coils a pass; R <= 3)
 bool tap_table_applies(const nufft3d_plan *p);
 // stored H (gather_tab.cu): plan-time build, and the gather of coils
 // c0..c0+cb-1 that reads it (cb 1, 2, 4 or 8; all coils of an odd count below

@@ -41,8 +41,8 @@ __device__ __forceinline__ void reduce_store(double acc, double *out)
 
 // Sum of a coil's partials, in every lane of its warp.  The scalar kernels run
 // a warp a coil: one thread adding the 304 partials waited on its chain of
-// loads and FP64 sums (13.9 us a kernel, twice an iteration; CG
-// of 8 iterations at 64^3 2289 -> 2135 us).
+// loads and FP64 sums (13.9 us a kernel; a CG iteration runs two of them; CG of 8
+// iterations at 64^3 2289 -> 2135 us).
 __device__ __forceinline__ double sum_parts(const double *parts, int c)
 {
     double s = 0;

@@ -17,8 +17,10 @@
 // overlap).  No shared-memory atomics, no kernel evaluation, and FP32
 // accumulation throughout.
 //
-// Measured at 128^3 x 8 coils: 2.39 ms (a row a grid point: 2.81 ms), of which
-// about 0.7 ms are the grid's atomics; 4 coils on 100 x 84 x 60 0.16 ms and one
+// Measured at 128^3 x 8 coils: 2.41 ms (a row a grid point: 2.81 ms), of which
+// about 0.7 ms are the grid's atomics (a copy without them); no unit is above
+// 52 % of its peak in a capture at 96^3, the warps wait at a piece's barriers
+// (the runs end at different times) and on lines and atomics; 4 coils on 100 x 84 x 60 0.16 ms and one
 // coil at 64^3 0.08 ms, where the spread evaluated the kernel before (0.46 and
 // 0.24 ms).  A lane for a whole row (8 coils x 4 points: 64 accumulators, code
 // that overflows the instruction cache when the loads are unrolled) took
@@ -457,8 +459,8 @@ __device__ __forceinline__ void stage_samples(const float2 *__restrict__ ks, int
 // are added to the grid.  The lines end with a spare step, so the loads that run
 // ahead need no bounds test.
 //
-// The vector atomics leave an SM at about 50 G requests a second in all,
-// whatever their width (a request is what one warp instruction adds to one
+// The vector atomics leave the chip at about 50 G requests a second (timed by
+// themselves), whatever their width (a request is what one warp instruction adds to one
 // 128-byte line), so the four rows of eight lanes exchange their 16-byte parts
 // first and each instruction adds whole points: two neighbouring points of 8
 // coils, 128 bytes, a request.
